@@ -1,4 +1,5 @@
-"""ctypes binding of ``libwtconv_b200.so`` (the C ABI in ``include/wtconv_b200.h``).
+"""Bindings of ``libwtconv_b200.so``: ctypes for the C ABI in ``include/wtconv_b200.h``, and the native
+host path the modules call.
 
 The shared library holds the hand-written sm_100a kernels; there is no other
 implementation behind this module.  If the library has not been built the import
@@ -18,6 +19,7 @@ F32, BF16, F16 = 0, 1, 2
 
 _lock = threading.Lock()
 _lib = None
+_host = None
 
 # every symbol include/wtconv_b200.h declares: (name, restype, argtypes)
 _VP, _I, _LLP = ctypes.c_void_p, ctypes.c_int, ctypes.POINTER(ctypes.c_longlong)
@@ -68,6 +70,22 @@ def load():
                 fn.argtypes = args
             _lib = lib
     return _lib
+
+
+def host():
+    """The native host path of the modules (``_host``, built from csrc/torch_host.cpp), which calls the
+    library above; raises WTConvLibraryError when it is not built."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise WTConvLibraryError(
+                "wtconv_b200/_host is missing or does not load: build it first (python -m wtconv_b200.build, or "
+                "__graft_entry__.build()). There is no fallback implementation.") from e
+        _host = module
+    return _host
 
 
 def status_string(status: int) -> str:

@@ -1,0 +1,568 @@
+// Host path of the modules: everything a layer call does between Python and the C ABI.
+//
+// A call of a small layer is a few microseconds of kernels; as Python (attribute walks over the
+// parameters, ctypes argument conversion, autograd.Function) the same call took 30 us for an
+// inference forward and 450 us for a training step, most of it spent before the first launch.  Here
+// the parameter walk reads the module dictionaries directly, the call geometry is kept per layer,
+// and the layer is a C++ autograd node, so the backward pass needs neither the interpreter nor its lock.
+//
+// Semantics are those of the reference modules (wtconv/wtconv2d.py:38-87, wtconv/wtconv1d.py:38-87) plus
+// their autograd: the input gradient is the layer run on the adjoint parameter block (the Haar transform
+// is orthogonal, odd sizes are padded and cropped at the same places), the parameter gradients are
+// correlation sums between sub-band pyramids.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <ATen/cuda/CUDAGraphsUtils.cuh>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/utils/object_ptr.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <array>
+#include <memory>
+#include <mutex>
+#include <string>
+#include <vector>
+
+#include "../../include/wtconv_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::variable_list;
+
+[[noreturn]] void fail(int status, const char* what) {
+  const std::string msg = std::string(what) + ": " + wtconv_status_string(status) + " (status " + std::to_string(status) + ")";
+  if (status == WTCONV_ERR_BAD_KERNEL_SIZE || status == WTCONV_ERR_BAD_LEVELS) C10_THROW_ERROR(ValueError, msg);
+  throw std::runtime_error(msg);
+}
+inline void check(int status, const char* what) {
+  if (status) fail(status, what);
+}
+
+int dtype_code(at::ScalarType t) {
+  switch (t) {
+    case at::kFloat: return WTCONV_F32;
+    case at::kBFloat16: return WTCONV_BF16;
+    case at::kHalf: return WTCONV_F16;
+    default: return -1;
+  }
+}
+
+// What a call needs to know about its layer: the geometry attributes and the parameters
+// [base weight, base bias (may be undefined), base scale, (wavelet weight, wavelet scale) per level].
+struct LayerDesc {
+  int ndim = 2, C = 0, K = 0, L = 0, stride = 1;
+  at::ScalarType filter_dtype = at::kFloat;
+  std::vector<Tensor> params;
+  std::string master_key;        // nn.DataParallel replicas: key of the master's parameters
+};
+
+// Tap magnitude exactly as a reference module of this dtype stores it in wt_filter / iwt_filter
+double tap_magnitude(int ndim, at::ScalarType t) {
+  const float s = static_cast<float>(0.70710678118654752440);
+  const float v = ndim == 2 ? s * s : s;
+  if (t == at::kBFloat16) return static_cast<float>(c10::BFloat16(v));
+  if (t == at::kHalf) return static_cast<float>(c10::Half(v));
+  return v;
+}
+
+// Identity of the parameter values: storage, address, in-place version, dtypes
+std::string param_key(const LayerDesc& d) {
+  std::string key;
+  key.reserve(d.params.size() * 24 + 8);
+  auto put = [&](const void* p, size_t n) { key.append(static_cast<const char*>(p), n); };
+  for (const Tensor& p : d.params) {
+    uint64_t w[3] = {0, 0, 0};
+    if (p.defined()) {
+      w[0] = reinterpret_cast<uint64_t>(p.unsafeGetTensorImpl()->unsafe_storage().unsafeGetStorageImpl());
+      w[1] = reinterpret_cast<uint64_t>(p.const_data_ptr());
+      w[2] = p._version();
+    }
+    put(w, sizeof(w));
+  }
+  const int8_t t[2] = {static_cast<int8_t>(d.params[0].scalar_type()), static_cast<int8_t>(d.filter_dtype)};
+  put(t, sizeof(t));
+  return key;
+}
+
+// Folded parameter block of one (device, adjoint) pair
+struct Packed {
+  int device = -1;
+  bool adjoint = false;
+  std::string key;
+  Tensor block;
+  std::shared_ptr<at::cuda::CUDAEvent> written;
+  std::vector<cudaStream_t> seen;       // streams that wrote the block or waited for it
+};
+
+// Geometry of a 2-D call: output layout, stride arrays, scratch bytes
+struct Plan {
+  std::array<int64_t, 4> sizes, strides;
+  at::ScalarType dtype;
+  int stride;
+  bool make_contiguous;
+  at::MemoryFormat format;
+  std::array<int64_t, 4> out;
+  long long xs[4], ys[4];
+  size_t ws_bytes;
+};
+
+// State of one layer (and of its replicas): folded blocks and call geometries.  Calls may come from
+// several host threads (nn.DataParallel, autograd workers).
+class LayerState {
+ public:
+  // Folded block for the parameters' current values, ready on the current stream of `device`.
+  Tensor packed(const LayerDesc& d, c10::Device device, bool adjoint) {
+    const std::string key = d.master_key.empty() ? param_key(d) : d.master_key;
+    const c10::cuda::CUDAStream cur = c10::cuda::getCurrentCUDAStream(device.index());
+    std::lock_guard<std::mutex> lock(mu_);
+    Packed* slot = nullptr;
+    for (Packed& p : blocks_)
+      if (p.device == device.index() && p.adjoint == adjoint) slot = &p;
+    if (slot && slot->key == key) {
+      // the block was written on the stream that was current at the time: other streams wait once
+      bool known = false;
+      for (cudaStream_t s : slot->seen) known = known || s == cur.stream();
+      if (!known && at::cuda::currentStreamCaptureStatusMayInitCtx() == at::cuda::CaptureStatus::None) {
+        slot->written->block(cur);
+        c10::cuda::CUDACachingAllocator::recordStream(slot->block.storage().data_ptr(), cur);
+        slot->seen.push_back(cur.stream());
+      }
+      return slot->block;
+    }
+    Packed fresh = fold(d, device, adjoint, cur);
+    fresh.key = key;
+    Tensor block = fresh.block;
+    if (slot) *slot = std::move(fresh);
+    else blocks_.push_back(std::move(fresh));
+    return block;
+  }
+
+  // Geometry of a call on `x` (contiguous copies are planned for, not made, here)
+  Plan plan(const LayerDesc& d, const Tensor& x, int stride) {
+    const auto sz = x.sizes();
+    const auto st = x.strides();
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      for (const Plan& p : plans_)
+        if (p.dtype == x.scalar_type() && p.stride == stride && std::equal(sz.begin(), sz.end(), p.sizes.begin()) &&
+            std::equal(st.begin(), st.end(), p.strides.begin()))
+          return p;
+    }
+    Plan p;
+    std::copy(sz.begin(), sz.end(), p.sizes.begin());
+    std::copy(st.begin(), st.end(), p.strides.begin());
+    p.dtype = x.scalar_type();
+    p.stride = stride;
+    const bool contiguous = x.is_contiguous();
+    const bool channels_last = !contiguous && x.is_contiguous(at::MemoryFormat::ChannelsLast);
+    p.make_contiguous = !contiguous && !channels_last;
+    p.format = channels_last ? at::MemoryFormat::ChannelsLast : at::MemoryFormat::Contiguous;
+    p.out = {sz[0], sz[1], (sz[2] + stride - 1) / stride, (sz[3] + stride - 1) / stride};
+    auto dense = [&](const std::array<int64_t, 4>& s, long long* o) {
+      if (channels_last) { o[0] = s[1] * s[2] * s[3]; o[1] = 1; o[2] = s[3] * s[1]; o[3] = s[1]; }
+      else { o[0] = s[1] * s[2] * s[3]; o[1] = s[2] * s[3]; o[2] = s[3]; o[3] = 1; }
+    };
+    if (p.make_contiguous) dense(p.sizes, p.xs);
+    else std::copy(st.begin(), st.end(), p.xs);
+    dense(p.out, p.ys);
+    p.ws_bytes = 0;
+    check(wtconv2d_workspace_bytes((int)sz[0], (int)sz[1], (int)sz[2], (int)sz[3], d.K, d.L, dtype_code(p.dtype), p.xs, p.ys,
+                                   &p.ws_bytes), "wtconv2d_workspace_bytes");
+    std::lock_guard<std::mutex> lock(mu_);
+    if (plans_.size() >= 64) plans_.clear();
+    plans_.push_back(p);
+    return p;
+  }
+
+ private:
+  static Packed fold(const LayerDesc& d, c10::Device device, bool adjoint, const c10::cuda::CUDAStream& cur) {
+    at::ScalarType pdt = at::ScalarType::Undefined;
+    std::vector<Tensor> hold;                       // contiguous views, alive until the launch has been enqueued
+    for (const Tensor& p : d.params) {
+      if (!p.defined()) { hold.emplace_back(); continue; }
+      if (pdt == at::ScalarType::Undefined) pdt = p.scalar_type();
+      if (p.scalar_type() != pdt || dtype_code(pdt) < 0)
+        throw torch::TypeError("WTConv parameters must share one dtype out of float32 / bfloat16 / float16");
+    }
+    for (const Tensor& p : d.params)
+      if (p.defined() && p.device() != device)
+        throw std::runtime_error("WTConv parameters and input must live on the same CUDA device");
+    hold.clear();
+    for (const Tensor& p : d.params) hold.push_back(p.defined() ? p.detach().contiguous() : Tensor());
+    Packed out;
+    out.device = device.index();
+    out.adjoint = adjoint;
+    const size_t n = wtconv_packed_param_floats(d.ndim, d.C, d.K, d.L);
+    out.block = at::detail::empty_cuda({(int64_t)n}, at::kFloat, device, std::nullopt);
+    const double tap = tap_magnitude(d.ndim, d.filter_dtype);
+    std::vector<const void*> ww(std::max(d.L, 1)), ws(std::max(d.L, 1));
+    for (int i = 0; i < d.L; ++i) { ww[i] = hold[3 + 2 * i].const_data_ptr(); ws[i] = hold[4 + 2 * i].const_data_ptr(); }
+    auto pack = adjoint ? wtconv_pack_params_adjoint : wtconv_pack_params;
+    check(pack(d.ndim, d.C, d.K, d.L, dtype_code(pdt), tap, tap, hold[0].const_data_ptr(),
+               hold[1].defined() ? hold[1].const_data_ptr() : nullptr, hold[2].const_data_ptr(), ww.data(), ws.data(),
+               out.block.data_ptr<float>(), cur.stream()), "wtconv_pack_params");
+    out.written = std::make_shared<at::cuda::CUDAEvent>();
+    out.written->record(cur);
+    out.seen.push_back(cur.stream());
+    return out;
+  }
+
+  std::mutex mu_;
+  std::vector<Packed> blocks_;
+  std::vector<Plan> plans_;
+};
+
+void check_input(const LayerDesc& d, const Tensor& x) {
+  if (!x.is_cuda()) throw std::runtime_error("wtconv_b200 layers run only on CUDA tensors (sm_100a kernels, no CPU path)");
+  if (dtype_code(x.scalar_type()) < 0)
+    throw torch::TypeError(std::string("unsupported activation dtype ") + c10::toString(x.scalar_type()) +
+                           "; use float32, bfloat16 or float16");
+  if (x.dim() != d.ndim + 2 || x.size(1) != d.C) {
+    std::string shape;
+    for (int64_t s : x.sizes()) shape += (shape.empty() ? "" : ", ") + std::to_string(s);
+    C10_THROW_ERROR(ValueError, "expected a " + std::to_string(d.ndim + 2) + "-D input with " + std::to_string(d.C) +
+                                    " channels, got (" + shape + ")");
+  }
+}
+
+// One pass of the layer (adjoint: with the flipped, bias-free block) on the current stream of x's device
+Tensor run2d(LayerState& st, const LayerDesc& d, const Tensor& xin, bool adjoint, int stride) {
+  if (xin.numel() == 0)
+    return xin.new_empty({xin.size(0), xin.size(1), (xin.size(2) + stride - 1) / stride, (xin.size(3) + stride - 1) / stride});
+  const c10::cuda::CUDAGuard guard(xin.device());
+  const Plan p = st.plan(d, xin, stride);
+  const Tensor x = p.make_contiguous ? xin.contiguous() : xin;
+  Tensor y = at::detail::empty_cuda(p.out, p.dtype, xin.device(), p.format);
+  const Tensor packed = st.packed(d, xin.device(), adjoint);
+  c10::DataPtr ws;
+  if (p.ws_bytes) ws = c10::cuda::CUDACachingAllocator::get()->allocate(p.ws_bytes);
+  check(wtconv2d_forward(x.const_data_ptr(), y.data_ptr(), packed.const_data_ptr<float>(), ws.get(), p.ws_bytes,
+                         (int)p.sizes[0], (int)p.sizes[1], (int)p.sizes[2], (int)p.sizes[3], d.K, d.L, stride,
+                         dtype_code(p.dtype), p.xs, p.ys, c10::cuda::getCurrentCUDAStream(xin.device().index()).stream()),
+        "wtconv2d_forward");
+  return y;
+}
+
+Tensor run1d(LayerState& st, const LayerDesc& d, const Tensor& xin, bool adjoint, int stride) {
+  const int64_t B = xin.size(0), C = xin.size(1), N = xin.size(2);
+  const c10::cuda::CUDAGuard guard(xin.device());
+  Tensor y = at::detail::empty_cuda({B, C, N / stride}, xin.scalar_type(), xin.device(), std::nullopt);
+  if (y.numel() == 0) return y;
+  const Tensor x = xin.stride(2) == 1 ? xin : xin.contiguous();
+  const Tensor packed = st.packed(d, xin.device(), adjoint);
+  const long long xs[3] = {x.stride(0), x.stride(1), x.stride(2)}, ys[3] = {y.stride(0), y.stride(1), y.stride(2)};
+  check(wtconv1d_forward(x.const_data_ptr(), y.data_ptr(), packed.const_data_ptr<float>(), (int)B, (int)C, (int)N, d.K, d.L,
+                         stride, dtype_code(x.scalar_type()), xs, ys,
+                         c10::cuda::getCurrentCUDAStream(xin.device().index()).stream()), "wtconv1d_forward");
+  return y;
+}
+
+Tensor run(LayerState& st, const LayerDesc& d, const Tensor& x, bool adjoint, int stride) {
+  return d.ndim == 2 ? run2d(st, d, x, adjoint, stride) : run1d(st, d, x, adjoint, stride);
+}
+
+// Adjoint of the output stride: the gradient of the layer output before the stride
+Tensor grad_to_full_resolution(const LayerDesc& d, const Tensor& gy, at::IntArrayRef in_shape) {
+  const int64_t s = d.stride;
+  if (s == 1) return gy;
+  Tensor full = at::zeros(in_shape, gy.options());
+  if (d.ndim == 2) {
+    full.slice(2, 0, std::nullopt, s).slice(3, 0, std::nullopt, s).copy_(gy);        // wtconv2d.py:33-34: AvgPool2d(1, s) picks samples
+  } else {
+    full.slice(2, 0, gy.size(2) * s).copy_(gy.repeat_interleave(s, -1).div_(static_cast<double>(s)));   // wtconv1d.py:34: AvgPool1d(s, s)
+  }
+  return full;
+}
+
+// Gradients of all parameters for input x and output gradient g (full resolution).  A 1-D signal is
+// handed to the 2-D kernels as a one-row image.
+variable_list param_grads(const LayerDesc& d, const Tensor& x, Tensor g) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  if (g.scalar_type() != x.scalar_type()) g = g.to(x.scalar_type());
+  const int B = (int)x.size(0), C = (int)x.size(1), K = d.K, L = d.L, code = dtype_code(x.scalar_type());
+  const int H = d.ndim == 2 ? (int)x.size(2) : 1, W = (int)x.size(d.ndim == 2 ? 3 : 2);
+  auto strides = [&](const Tensor& t, long long* s) {
+    s[0] = t.stride(0); s[1] = t.stride(1);
+    s[2] = d.ndim == 2 ? t.stride(2) : 0;
+    s[3] = t.stride(d.ndim == 2 ? 3 : 2);
+  };
+  long long xs[4], gs[4];
+  strides(x, xs);
+  strides(g, gs);
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
+  auto floats = [&](size_t n) { return at::detail::empty_cuda({(int64_t)std::max<size_t>(n, 1)}, at::kFloat, x.device(), std::nullopt); };
+  const size_t n = wtconv2d_pyramid_floats(B, C, H, W, L);
+  Tensor xp = floats(n), gp = floats(n), stats = floats(wtconv2d_weight_grad_stat_floats(C, K, L));
+  check(wtconv2d_pyramid(x.const_data_ptr(), xp.data_ptr<float>(), B, C, H, W, L, code, xs, stream), "wtconv2d_pyramid");
+  check(wtconv2d_pyramid(g.const_data_ptr(), gp.data_ptr<float>(), B, C, H, W, L, code, gs, stream), "wtconv2d_pyramid");
+  check(wtconv2d_weight_grad_stats(x.const_data_ptr(), g.const_data_ptr(), xp.data_ptr<float>(), gp.data_ptr<float>(),
+                                   stats.data_ptr<float>(), B, C, H, W, K, L, code, xs, gs, stream),
+        "wtconv2d_weight_grad_stats");
+  std::vector<Tensor> hold;
+  variable_list grads;
+  for (const Tensor& p : d.params) {
+    hold.push_back(p.defined() ? p.detach().contiguous() : Tensor());
+    grads.push_back(p.defined() ? at::empty_like(hold.back(), at::MemoryFormat::Contiguous) : Tensor());
+  }
+  const double tap = tap_magnitude(d.ndim, d.filter_dtype);
+  std::vector<const void*> ww(std::max(L, 1)), ws(std::max(L, 1));
+  std::vector<void*> gw(std::max(L, 1)), gsc(std::max(L, 1));
+  for (int i = 0; i < L; ++i) {
+    ww[i] = hold[3 + 2 * i].const_data_ptr(); ws[i] = hold[4 + 2 * i].const_data_ptr();
+    gw[i] = grads[3 + 2 * i].data_ptr(); gsc[i] = grads[4 + 2 * i].data_ptr();
+  }
+  check(wtconv_param_grads(d.ndim, C, K, L, dtype_code(hold[0].scalar_type()), tap, tap, stats.const_data_ptr<float>(),
+                           hold[0].const_data_ptr(), hold[1].defined() ? hold[1].const_data_ptr() : nullptr,
+                           hold[2].const_data_ptr(), ww.data(), ws.data(), grads[0].data_ptr(),
+                           grads[1].defined() ? grads[1].data_ptr() : nullptr, grads[2].data_ptr(), gw.data(), gsc.data(), stream),
+        "wtconv_param_grads");
+  return grads;
+}
+
+// The layer as one autograd node: inputs are x and the defined parameters, in order
+struct WTConvBackward : public torch::autograd::Node {
+  std::shared_ptr<LayerState> state;
+  LayerDesc desc;
+  torch::autograd::SavedVariable x;
+
+  std::string name() const override { return "WTConvBackward"; }
+
+  variable_list apply(variable_list&& grads) override {
+    const size_t nparam = num_outputs() - 1;
+    variable_list out(nparam + 1);
+    if (!grads[0].defined()) return out;
+    const bool twice = at::GradMode::is_enabled();
+    {
+      at::AutoGradMode off(false);
+      const Tensor xin = x.unpack(shared_from_this());
+      const Tensor g = grad_to_full_resolution(desc, grads[0], xin.sizes());
+      if (task_should_compute_output(0)) out[0] = run(*state, desc, g, true, 1);
+      bool any = false;
+      for (size_t i = 1; i <= nparam; ++i) any = any || task_should_compute_output(i);
+      if (any) {
+        variable_list all = param_grads(desc, xin, g);
+        size_t k = 1;
+        for (size_t i = 0; i < all.size(); ++i) {
+          if (!desc.params[i].defined()) continue;
+          if (task_should_compute_output(k)) out[k] = std::move(all[i]);
+          ++k;
+        }
+      }
+    }
+    if (twice) {
+      // create_graph: the gradients exist, differentiating them raises (torch.autograd.function.once_differentiable)
+      variable_list marked;
+      for (Tensor& t : out) {
+        if (t.defined()) { t = t.detach(); t.set_requires_grad(true); }
+        marked.push_back(t);
+      }
+      std::shared_ptr<torch::autograd::Node> err(
+          new torch::autograd::DelayedError("trying to differentiate twice a function that was marked with @once_differentiable",
+                                            (int64_t)marked.size()),
+          torch::autograd::deleteNode);
+      out = (*err)(std::move(marked));
+    }
+    return out;
+  }
+
+  void release_variables() override { x.reset_data(); }
+};
+
+// ---------------------------------------------------------------------------
+// Python side
+// ---------------------------------------------------------------------------
+struct Names {
+  PyObject *modules, *parameters, *weight, *bias, *base_conv, *base_scale, *wavelet_convs, *wavelet_scale, *in_channels,
+      *kernel_size, *wt_levels, *stride, *wt_filter, *ndim, *native, *master_key;
+};
+const Names& names() {
+  static const Names n = {
+      PyUnicode_InternFromString("_modules"), PyUnicode_InternFromString("_parameters"), PyUnicode_InternFromString("weight"),
+      PyUnicode_InternFromString("bias"), PyUnicode_InternFromString("base_conv"), PyUnicode_InternFromString("base_scale"),
+      PyUnicode_InternFromString("wavelet_convs"), PyUnicode_InternFromString("wavelet_scale"),
+      PyUnicode_InternFromString("in_channels"), PyUnicode_InternFromString("kernel_size"),
+      PyUnicode_InternFromString("wt_levels"), PyUnicode_InternFromString("stride"), PyUnicode_InternFromString("wt_filter"),
+      PyUnicode_InternFromString("_ndim"), PyUnicode_InternFromString("_native"), PyUnicode_InternFromString("_master_key")};
+  return n;
+}
+
+typedef THPObjectPtr Ref;
+
+// obj.<dict_name>[key] when it is there, else getattr(obj, key) (parametrised or replaced attributes)
+PyObject* lookup(PyObject* obj, PyObject* dict_name, PyObject* key) {
+  Ref dict(PyObject_GetAttr(obj, dict_name));
+  if (!dict) throw python_error();
+  if (PyDict_Check(dict.get())) {
+    PyObject* v = PyDict_GetItemWithError(dict.get(), key);
+    if (v) { Py_INCREF(v); return v; }
+    if (PyErr_Occurred()) throw python_error();
+  }
+  PyObject* v = PyObject_GetAttr(obj, key);
+  if (!v) throw python_error();
+  return v;
+}
+
+Tensor tensor_of(PyObject* obj, bool allow_none) {
+  if (THPVariable_Check(obj)) return THPVariable_Unpack(obj);
+  if (allow_none && obj == Py_None) return Tensor();
+  throw torch::TypeError("WTConv parameters must be tensors");
+}
+Tensor param_of(PyObject* module, PyObject* key, bool allow_none = false) {
+  Ref v(lookup(module, names().parameters, key));
+  return tensor_of(v.get(), allow_none);
+}
+int int_attr(PyObject* obj, PyObject* key) {
+  Ref v(PyObject_GetAttr(obj, key));
+  if (!v) throw python_error();
+  const long n = PyLong_AsLong(v.get());
+  if (n == -1 && PyErr_Occurred()) throw python_error();
+  return (int)n;
+}
+
+LayerDesc describe(PyObject* self) {
+  const Names& n = names();
+  LayerDesc d;
+  d.ndim = int_attr(self, n.ndim);
+  d.C = int_attr(self, n.in_channels);
+  d.K = int_attr(self, n.kernel_size);
+  d.L = int_attr(self, n.wt_levels);
+  d.stride = int_attr(self, n.stride);
+  d.params.reserve(3 + 2 * d.L);
+  {
+    Ref conv(lookup(self, n.modules, n.base_conv));
+    d.params.push_back(param_of(conv.get(), n.weight));
+    d.params.push_back(param_of(conv.get(), n.bias, true));
+    Ref scale(lookup(self, n.modules, n.base_scale));
+    d.params.push_back(param_of(scale.get(), n.weight));
+  }
+  Ref convs(lookup(self, n.modules, n.wavelet_convs)), scales(lookup(self, n.modules, n.wavelet_scale));
+  Ref cd(PyObject_GetAttr(convs.get(), n.modules)), sd(PyObject_GetAttr(scales.get(), n.modules));
+  if (!cd || !sd) throw python_error();
+  Py_ssize_t ci = 0, si = 0;
+  PyObject *key, *conv, *scale;
+  for (int l = 0; l < d.L; ++l) {
+    if (!PyDict_Next(cd.get(), &ci, &key, &conv) || !PyDict_Next(sd.get(), &si, &key, &scale))
+      throw std::runtime_error("WTConv: fewer wavelet_convs / wavelet_scale modules than wt_levels");
+    Ref hc(conv), hs(scale);                        // keep the modules alive: getattr may run Python code
+    Py_INCREF(conv);
+    Py_INCREF(scale);
+    d.params.push_back(param_of(conv, n.weight));
+    d.params.push_back(param_of(scale, n.weight));
+  }
+  d.filter_dtype = param_of(self, n.wt_filter).scalar_type();
+  return d;
+}
+
+// Attribute that may be absent, without raising through nn.Module.__getattr__
+PyObject* instance_item(PyObject* self, PyObject* key) {
+  Ref dict(PyObject_GenericGetDict(self, nullptr));
+  if (!dict) throw python_error();
+  PyObject* v = PyDict_GetItemWithError(dict.get(), key);
+  if (!v && PyErr_Occurred()) throw python_error();
+  return v;
+}
+
+std::shared_ptr<LayerState> state_of(PyObject* self) {
+  PyObject* v = instance_item(self, names().native);
+  if (v && v != Py_None) return py::cast<std::shared_ptr<LayerState>>(py::handle(v));
+  auto st = std::make_shared<LayerState>();
+  py::object o = py::cast(st);
+  if (PyObject_SetAttr(self, names().native, o.ptr())) throw python_error();
+  return st;
+}
+
+void take_master_key(PyObject* self, LayerDesc& d) {
+  PyObject* v = instance_item(self, names().master_key);
+  if (v && PyBytes_Check(v)) d.master_key.assign(PyBytes_AS_STRING(v), PyBytes_GET_SIZE(v));
+}
+
+// forward(module, x)
+PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 2 || !THPVariable_Check(args[1])) throw torch::TypeError("expected a module and a tensor");
+  PyObject* self = args[0];
+  const Tensor x = THPVariable_Unpack(args[1]);
+  LayerDesc d = describe(self);
+  check_input(d, x);
+  take_master_key(self, d);
+  const std::shared_ptr<LayerState> st = state_of(self);
+  bool needs = false;
+  if (at::GradMode::is_enabled()) {
+    needs = x.requires_grad();
+    for (const Tensor& p : d.params) needs = needs || (p.defined() && p.requires_grad());
+  }
+  Tensor y;
+  {
+    pybind11::gil_scoped_release no_gil;
+    if (!needs) {
+      y = run(*st, d, x, false, d.stride);
+    } else {
+      {
+        at::AutoGradMode off(false);
+        y = run(*st, d, x, false, d.stride);
+      }
+      std::shared_ptr<WTConvBackward> node(new WTConvBackward(), torch::autograd::deleteNode);
+      torch::autograd::edge_list edges;
+      edges.push_back(torch::autograd::impl::gradient_edge(x));
+      for (const Tensor& p : d.params)
+        if (p.defined()) edges.push_back(torch::autograd::impl::gradient_edge(p));
+      node->set_next_edges(std::move(edges));
+      node->state = st;
+      node->x = torch::autograd::SavedVariable(x, false);
+      node->desc = std::move(d);
+      torch::autograd::set_history(y, node);
+    }
+  }
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
+// packed(module, device, adjoint)
+PyObject* py_packed(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 3) throw torch::TypeError("expected a module, a device and a flag");
+  LayerDesc d = describe(args[0]);
+  take_master_key(args[0], d);
+  c10::Device dev = py::cast<c10::Device>(py::handle(args[1]));
+  if (!dev.has_index()) dev = c10::Device(dev.type(), c10::cuda::current_device());
+  const c10::cuda::CUDAGuard guard(dev);
+  return THPVariable_Wrap(state_of(args[0])->packed(d, dev, PyObject_IsTrue(args[2]) == 1));
+  END_HANDLE_TH_ERRORS
+}
+
+// param_key(module)
+PyObject* py_param_key(PyObject*, PyObject* self) {
+  HANDLE_TH_ERRORS
+  const std::string k = param_key(describe(self));
+  return PyBytes_FromStringAndSize(k.data(), (Py_ssize_t)k.size());
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef kMethods[] = {
+    {"forward", (PyCFunction)(void (*)(void))py_forward, METH_FASTCALL, "One call of a layer, with autograd."},
+    {"packed", (PyCFunction)(void (*)(void))py_packed, METH_FASTCALL, "Folded parameter block of a layer on a device."},
+    {"param_key", (PyCFunction)py_param_key, METH_O, "Identity of a layer's parameter values."},
+    {nullptr, nullptr, 0, nullptr}};
+
+}  // namespace
+
+PYBIND11_MODULE(_host, m) {
+  // Copies and pickles of a module start with an empty state: the blocks are folded again on first use
+  py::class_<LayerState, std::shared_ptr<LayerState>>(m, "LayerState")
+      .def(py::init<>())
+      .def("__deepcopy__", [](const LayerState&, py::object) { return std::make_shared<LayerState>(); })
+      .def(py::pickle([](const LayerState&) { return py::tuple(); }, [](const py::tuple&) { return std::make_shared<LayerState>(); }));
+  if (PyModule_AddFunctions(m.ptr(), kMethods)) throw py::error_already_set();
+}
