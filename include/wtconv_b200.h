@@ -270,6 +270,22 @@ int wtconv1d_forward(const void* x, void* y, const float* packed,
                      int B, int C, int N, int K, int L, int stride, int dtype,
                      const long long* x_strides, const long long* y_strides, void* stream);
 
+/*
+ * Backward pass of WTConv1d without intermediates in memory, for kernel sizes 1, 3, 5, 7, up to five
+ * levels and unit time strides (WTCONV_ERR_BAD_LEVELS otherwise; the one-row-image path of
+ * wtconv2d_weight_grad_stats covers the rest).
+ *
+ * wtconv1d_input_grad: gradient of the input (B,C,N) from gy (B,C,floor(N/stride)); the spreading of a
+ * pooled gradient over its `stride` samples (wtconv1d.py:34) happens while loading.  packed_adjoint is
+ * the block of wtconv_pack_params_adjoint.
+ * wtconv1d_weight_grad_stats: the correlation sums wtconv_param_grads (ndim = 1) reads, in the layout
+ * and size of wtconv2d_weight_grad_stats; zeroed by the call.
+ */
+int wtconv1d_input_grad(const void* gy, void* gx, const float* packed_adjoint, int B, int C, int N, int K, int L,
+                        int stride, int dtype, const long long* g_strides, const long long* x_strides, void* stream);
+int wtconv1d_weight_grad_stats(const void* x, const void* gy, float* stats, int B, int C, int N, int K, int L,
+                               int stride, int dtype, const long long* x_strides, const long long* g_strides, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -43,6 +43,8 @@ SYMBOLS = {
     "wtconv2d_launch_count": (_I, [_I, _I, _I, _I, _I, _I, _I, _I, _LLP, _LLP, ctypes.POINTER(_I)]),
     "wtconv2d_forward": (_I, [_VP, _VP, _VP, _VP, ctypes.c_size_t, _I, _I, _I, _I, _I, _I, _I, _I, _LLP, _LLP, _VP]),
     "wtconv2d_forward_noalloc": (_I, [_VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _I, _I, _LLP, _LLP, _VP]),
+    "wtconv1d_input_grad": (_I, [_VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _I, _LLP, _LLP, _VP]),
+    "wtconv1d_weight_grad_stats": (_I, [_VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _I, _LLP, _LLP, _VP]),
     "wtconv1d_forward": (_I, [_VP, _VP, _VP, _I, _I, _I, _I, _I, _I, _I, _LLP, _LLP, _VP]),
 }
 

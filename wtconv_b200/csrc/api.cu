@@ -512,10 +512,11 @@ int wtconv1d_forward(const void* x, void* y, const float* packed, int B, int C, 
     if (ly.xs[i] < 0 || ly.ys[i] < 0) return WTCONV_ERR_BAD_ARG;
   }
   if (wt1d_warp_supported(K, L, stride, ly.xs[2], ly.ys[2])) {
-    // time-contiguous signals, stride 1, up to four levels: the register-resident kernel
+    // time-contiguous signals, up to five levels: the register-resident kernel
     Warp1dArgs wa;
     wa.x = x; wa.y = y; wa.packed = packed;
     wa.B = B; wa.C = C; wa.N = N;
+    wa.pool = stride; wa.up = 1;
     wa.wstride = packed_channel_floats(K, 1, L);
     wa.nseg = 0; wa.nwarps = 0;
     wa.xs0 = ly.xs[0]; wa.xs1 = ly.xs[1]; wa.ys0 = ly.ys[0]; wa.ys1 = ly.ys[1];
@@ -528,6 +529,47 @@ int wtconv1d_forward(const void* x, void* y, const float* packed, int B, int C, 
   if (ps) return ps;
   if (p.ngroups > 65535) return WTCONV_ERR_TOO_LARGE;
   return (int)launch_wt1d(p, dtype, x, y, packed, (size_t)smem, static_cast<cudaStream_t>(stream));
+}
+
+int wtconv1d_input_grad(const void* gy, void* gx, const float* packed_adjoint, int B, int C, int N, int K, int L, int stride,
+                        int dtype, const long long* g_strides, const long long* x_strides, void* stream) {
+  if (!gy || !gx || !packed_adjoint) return WTCONV_ERR_BAD_ARG;
+  const int st = check_common(C, K, L, dtype);
+  if (st) return st;
+  if (B <= 0 || N <= 0 || stride < 1 || !g_strides || !x_strides) return WTCONV_ERR_BAD_ARG;
+  if (!wt1d_warp_levels(K, L) || g_strides[2] != 1 || x_strides[2] != 1) return WTCONV_ERR_BAD_LEVELS;
+  if (B > 65535 || (long long)C * N >= (1LL << 31) || (long long)B * C * N >= (1LL << 40)) return WTCONV_ERR_TOO_LARGE;
+  if (ptr_align(gy) < elem_size(dtype) || ptr_align(gx) < elem_size(dtype) || ptr_align(packed_adjoint) < 16)
+    return WTCONV_ERR_MISALIGNED;
+  Warp1dArgs a;
+  a.x = gy; a.y = gx; a.packed = packed_adjoint;
+  a.B = B; a.C = C; a.N = N;
+  a.pool = 1; a.up = stride;
+  a.wstride = packed_channel_floats(K, 1, L);
+  a.nseg = 0; a.nwarps = 0;
+  a.xs0 = g_strides[0]; a.xs1 = g_strides[1]; a.ys0 = x_strides[0]; a.ys1 = x_strides[1];
+  const cudaError_t e = launch_wt1d_warp(a, K, L, dtype, static_cast<cudaStream_t>(stream));
+  return e == cudaErrorNotSupported ? WTCONV_ERR_TOO_LARGE : (int)e;
+}
+
+int wtconv1d_weight_grad_stats(const void* x, const void* gy, float* stats, int B, int C, int N, int K, int L, int stride,
+                               int dtype, const long long* x_strides, const long long* g_strides, void* stream) {
+  if (!x || !gy || !stats) return WTCONV_ERR_BAD_ARG;
+  const int st = check_common(C, K, L, dtype);
+  if (st) return st;
+  if (B <= 0 || N <= 0 || stride < 1 || !g_strides || !x_strides) return WTCONV_ERR_BAD_ARG;
+  if (!unrolled_k(K)) return WTCONV_ERR_BAD_KERNEL_SIZE;
+  if (!wt1d_warp_levels(K, L) || g_strides[2] != 1 || x_strides[2] != 1) return WTCONV_ERR_BAD_LEVELS;
+  if ((long long)C * N >= (1LL << 31) || (long long)B * C * N >= (1LL << 40) || C > (1 << 20)) return WTCONV_ERR_TOO_LARGE;
+  cudaStream_t cs = static_cast<cudaStream_t>(stream);
+  cudaError_t e = cudaMemsetAsync(stats, 0, wtconv2d_weight_grad_stat_floats(C, K, L) * sizeof(float), cs);
+  if (e != cudaSuccess) return (int)e;
+  Wgrad1dArgs a;
+  a.x = x; a.g = gy; a.stats = stats;
+  a.B = B; a.C = C; a.N = N; a.up = stride;
+  a.nseg = a.nsplit = 0; a.items = 0;
+  a.xs0 = x_strides[0]; a.xs1 = x_strides[1]; a.gs0 = g_strides[0]; a.gs1 = g_strides[1];
+  return (int)launch_wt1d_wgrad(a, K, L, dtype, cs);
 }
 
 }  // extern "C"

@@ -269,6 +269,23 @@ Tensor run1d(LayerState& st, const LayerDesc& d, const Tensor& xin, bool adjoint
   return y;
 }
 
+// The 1-D backward kernels cover this call: kernel sizes with an unrolled instance, up to five levels,
+// contiguous samples in both tensors
+bool fused_backward_1d(const LayerDesc& d, const Tensor& x, const Tensor& gy) {
+  return d.ndim == 1 && d.L <= 5 && d.K <= 7 && x.stride(2) == 1 && gy.stride(2) == 1 && x.scalar_type() == gy.scalar_type();
+}
+
+Tensor input_grad_1d(LayerState& st, const LayerDesc& d, const Tensor& x, const Tensor& gy) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  Tensor gx = at::detail::empty_cuda(x.sizes(), x.scalar_type(), x.device(), std::nullopt);
+  const Tensor packed = st.packed(d, x.device(), true);
+  const long long gs[3] = {gy.stride(0), gy.stride(1), gy.stride(2)}, xs[3] = {gx.stride(0), gx.stride(1), gx.stride(2)};
+  check(wtconv1d_input_grad(gy.const_data_ptr(), gx.data_ptr(), packed.const_data_ptr<float>(), (int)x.size(0), d.C,
+                            (int)x.size(2), d.K, d.L, d.stride, dtype_code(x.scalar_type()), gs, xs,
+                            c10::cuda::getCurrentCUDAStream(x.device().index()).stream()), "wtconv1d_input_grad");
+  return gx;
+}
+
 Tensor run(LayerState& st, const LayerDesc& d, const Tensor& x, bool adjoint, int stride) {
   return d.ndim == 2 ? run2d(st, d, x, adjoint, stride) : run1d(st, d, x, adjoint, stride);
 }
@@ -286,11 +303,9 @@ Tensor grad_to_full_resolution(const LayerDesc& d, const Tensor& gy, at::IntArra
   return full;
 }
 
-// Gradients of all parameters for input x and output gradient g (full resolution).  A 1-D signal is
-// handed to the 2-D kernels as a one-row image.
-variable_list param_grads(const LayerDesc& d, const Tensor& x, Tensor g) {
-  const c10::cuda::CUDAGuard guard(x.device());
-  if (g.scalar_type() != x.scalar_type()) g = g.to(x.scalar_type());
+// Correlation sums for input x and output gradient g (full resolution).  A 1-D signal the fused kernel
+// does not cover is handed to the 2-D kernels as a one-row image.
+void grad_stats(const LayerDesc& d, const Tensor& x, const Tensor& g, Tensor& stats) {
   const int B = (int)x.size(0), C = (int)x.size(1), K = d.K, L = d.L, code = dtype_code(x.scalar_type());
   const int H = d.ndim == 2 ? (int)x.size(2) : 1, W = (int)x.size(d.ndim == 2 ? 3 : 2);
   auto strides = [&](const Tensor& t, long long* s) {
@@ -302,14 +317,20 @@ variable_list param_grads(const LayerDesc& d, const Tensor& x, Tensor g) {
   strides(x, xs);
   strides(g, gs);
   cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
-  auto floats = [&](size_t n) { return at::detail::empty_cuda({(int64_t)std::max<size_t>(n, 1)}, at::kFloat, x.device(), std::nullopt); };
-  const size_t n = wtconv2d_pyramid_floats(B, C, H, W, L);
-  Tensor xp = floats(n), gp = floats(n), stats = floats(wtconv2d_weight_grad_stat_floats(C, K, L));
+  const int64_t n = std::max<int64_t>((int64_t)wtconv2d_pyramid_floats(B, C, H, W, L), 1);
+  Tensor xp = at::detail::empty_cuda({n}, at::kFloat, x.device(), std::nullopt);
+  Tensor gp = at::detail::empty_cuda({n}, at::kFloat, x.device(), std::nullopt);
   check(wtconv2d_pyramid(x.const_data_ptr(), xp.data_ptr<float>(), B, C, H, W, L, code, xs, stream), "wtconv2d_pyramid");
   check(wtconv2d_pyramid(g.const_data_ptr(), gp.data_ptr<float>(), B, C, H, W, L, code, gs, stream), "wtconv2d_pyramid");
   check(wtconv2d_weight_grad_stats(x.const_data_ptr(), g.const_data_ptr(), xp.data_ptr<float>(), gp.data_ptr<float>(),
                                    stats.data_ptr<float>(), B, C, H, W, K, L, code, xs, gs, stream),
         "wtconv2d_weight_grad_stats");
+}
+
+// Gradients of all parameters from the correlation sums
+variable_list param_grads(const LayerDesc& d, const Tensor& stats) {
+  const int L = d.L;
+  cudaStream_t stream = c10::cuda::getCurrentCUDAStream(stats.device().index()).stream();
   std::vector<Tensor> hold;
   variable_list grads;
   for (const Tensor& p : d.params) {
@@ -323,7 +344,7 @@ variable_list param_grads(const LayerDesc& d, const Tensor& x, Tensor g) {
     ww[i] = hold[3 + 2 * i].const_data_ptr(); ws[i] = hold[4 + 2 * i].const_data_ptr();
     gw[i] = grads[3 + 2 * i].data_ptr(); gsc[i] = grads[4 + 2 * i].data_ptr();
   }
-  check(wtconv_param_grads(d.ndim, C, K, L, dtype_code(hold[0].scalar_type()), tap, tap, stats.const_data_ptr<float>(),
+  check(wtconv_param_grads(d.ndim, d.C, d.K, L, dtype_code(hold[0].scalar_type()), tap, tap, stats.const_data_ptr<float>(),
                            hold[0].const_data_ptr(), hold[1].defined() ? hold[1].const_data_ptr() : nullptr,
                            hold[2].const_data_ptr(), ww.data(), ws.data(), grads[0].data_ptr(),
                            grads[1].defined() ? grads[1].data_ptr() : nullptr, grads[2].data_ptr(), gw.data(), gsc.data(), stream),
@@ -347,12 +368,31 @@ struct WTConvBackward : public torch::autograd::Node {
     {
       at::AutoGradMode off(false);
       const Tensor xin = x.unpack(shared_from_this());
-      const Tensor g = grad_to_full_resolution(desc, grads[0], xin.sizes());
-      if (task_should_compute_output(0)) out[0] = run(*state, desc, g, true, 1);
+      const c10::cuda::CUDAGuard guard(xin.device());
       bool any = false;
       for (size_t i = 1; i <= nparam; ++i) any = any || task_should_compute_output(i);
+      Tensor stats;
+      if (any)
+        stats = at::detail::empty_cuda({(int64_t)wtconv2d_weight_grad_stat_floats(desc.C, desc.K, desc.L)}, at::kFloat,
+                                       xin.device(), std::nullopt);
+      const Tensor& gy = grads[0];
+      if (gy.numel() > 0 && fused_backward_1d(desc, xin, gy)) {
+        if (task_should_compute_output(0)) out[0] = input_grad_1d(*state, desc, xin, gy);
+        if (any) {
+          const long long xs[3] = {xin.stride(0), xin.stride(1), 1}, gs[3] = {gy.stride(0), gy.stride(1), 1};
+          check(wtconv1d_weight_grad_stats(xin.const_data_ptr(), gy.const_data_ptr(), stats.data_ptr<float>(), (int)xin.size(0),
+                                           desc.C, (int)xin.size(2), desc.K, desc.L, desc.stride,
+                                           dtype_code(xin.scalar_type()), xs, gs,
+                                           c10::cuda::getCurrentCUDAStream(xin.device().index()).stream()),
+                "wtconv1d_weight_grad_stats");
+        }
+      } else {
+        const Tensor g = grad_to_full_resolution(desc, gy, xin.sizes());
+        if (task_should_compute_output(0)) out[0] = run(*state, desc, g, true, 1);
+        if (any) grad_stats(desc, xin, g.scalar_type() == xin.scalar_type() ? g : g.to(xin.scalar_type()), stats);
+      }
       if (any) {
-        variable_list all = param_grads(desc, xin, g);
+        variable_list all = param_grads(desc, stats);
         size_t k = 1;
         for (size_t i = 0; i < all.size(); ++i) {
           if (!desc.params[i].defined()) continue;

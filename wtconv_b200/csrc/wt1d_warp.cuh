@@ -1,43 +1,53 @@
 // Register-resident WTConv1d forward for time-contiguous signals (sm_100a).
 //
 // Same arithmetic as the CTA-tile kernel of wt1d_fused.cuh (reference: wtconv/wtconv1d.py:38-87,
-// wtconv/util/wavelet.py:46-59) for the common case: stride 1, at most four levels, samples of a
-// row contiguous in memory.  Nothing but the staging of unaligned rows goes through shared memory:
+// wtconv/util/wavelet.py:46-59) for the common case: at most five levels, a stride of 1, 2, 4 or 8,
+// samples of a row contiguous in memory.
 //
-//   * a thread owns 16 consecutive samples of one row (one channel of one sample), so the whole
-//     analysis cascade of up to four levels (2-tap Haar steps, un-normalised: the tap magnitudes
-//     are folded into the packed taps) is local to the thread;
+//   * a thread owns SPT = 16 or 32 consecutive samples of one row (one channel of one sample), so
+//     the whole analysis cascade of up to log2(SPT) levels (2-tap Haar steps, un-normalised: the
+//     tap magnitudes are folded into the packed taps) is local to the thread;
 //   * the K-tap sub-band convolutions and the base convolution need K/2 neighbours per side and
 //     level: they come from the neighbouring lanes by warp shuffles;
 //   * the low-pass accumulation (wtconv1d.py:71) and the synthesis are pointwise, hence local;
-//   * a warp therefore handles 32 x 16 consecutive samples of which the outer HL lanes per side
-//     only supply neighbours (HL = ceil((K/2) * 2^L / 16): two lanes for K = 5, L = 4); consecutive
-//     warps of a row overlap by those lanes.  Samples outside the signal are zeros, which is both
-//     the right-hand zero padding of odd lengths at every level (wtconv1d.py:49-51) and the
-//     'same' padding of the convolutions;
-//   * the taps of the row's channel are the same for the whole warp: it copies them (at most 18
+//   * a warp therefore handles 32 x SPT consecutive samples of which the outer HL lanes per side
+//     only supply neighbours (HL = ceil((K/2) * 2^L / SPT): one lane for K = 5, L = 4, SPT = 32);
+//     consecutive warps of a row overlap by those lanes.  Samples outside the signal are zeros,
+//     which is both the right-hand zero padding of odd lengths at every level (wtconv1d.py:49-51)
+//     and the 'same' padding of the convolutions;
+//   * the taps of the row's channel are the same for the whole warp: it copies them (at most 22
 //     128-bit words) into shared memory while its samples are on their way and reads them back
 //     as broadcasts.
 //
-// Rows that start on a 16-byte boundary are read and written with 128-bit accesses (every byte of
-// a touched sector is used by the same lane); other rows are staged through a 2.5 KB per-warp
-// buffer with coalesced element-wise accesses.
+// Samples enter and leave through a per-warp staging buffer, because a thread's run is SPT samples
+// apart from its neighbour's: 128-bit accesses straight to global memory at that distance took one
+// cycle of the load/store pipe per sector (the pipe was 75 % busy, DRAM 55 %).  Rows that start on a
+// 16-byte boundary are copied in with 16-byte cp.async, other fp32 rows with 4-byte ones.  The buffer is
+// swizzled (warp1d_slot) so that both sides of the exchange are free of bank conflicts.
+//
+// wt1d_wgrad_kernel (parameter gradients) runs the same cascade on the input and on the output
+// gradient at once and keeps every correlation sum of a channel in registers.
 #pragma once
 
 #include "wt_common.h"
 
 namespace wt {
 
-constexpr int kWarp1dSpt = 16;        // samples per thread
-constexpr int kWarp1dPitch = 20;      // floats between the runs of two threads in the staging buffer
 constexpr int kWarp1dWarps = 8;       // warps per CTA
-constexpr int kWarp1dMaxLevels = 4;   // 2^4 = samples per thread
+constexpr int kWarp1dMaxLevels = 5;
+// lanes per side that only supply neighbours, and the samples a warp produces
+WT_HD constexpr int warp1d_halo(int K, int L, int SPT) { return ((K / 2) * (1 << L) + SPT - 1) / SPT; }
+WT_HD constexpr int warp1d_segment(int K, int L, int SPT) { return (32 - 2 * warp1d_halo(K, L, SPT)) * SPT; }
+// 128-bit words of a channel's tap sets
+WT_HD constexpr int warp1d_tap_words(int K, int L) { return (1 + 2 * L) * ((K + 1 + 3) / 4); }
 
 struct Warp1dArgs {
   const void* x;
   void* y;
   const float* packed;
   int B, C, N;
+  int pool;               // output stride: 1, or the average of 2, 4, 8 samples (wtconv1d.py:34)
+  int up;                 // 1, or the input is the gradient of an output with this stride: sample t is x[t / up] / up
   int wstride;            // floats per channel in the packed block
   int nseg;               // warps per row
   long long nwarps;       // rows * nseg
@@ -77,6 +87,79 @@ __device__ __forceinline__ void warp1d_conv(const float (&ext)[NJ + K - 1], cons
     for (int o = 0; o < NJ; ++o) acc[o] = fmaf(w[k], ext[o + k], acc[o]);
 }
 
+// Staging buffer of a warp: run r (lane r's samples) takes CPT 16-byte chunks; chunk c of run r is stored at
+// chunk c ^ (r / (8 / CPT)) of the run, so the eight lanes of a quarter warp, which touch the same chunk of
+// eight runs or eight consecutive chunks, always hit eight different 16-byte bank groups.
+// Byte offset of chunk k of this lane's run:
+template <typename T, int SPT>
+__device__ __forceinline__ int warp1d_own(int lane, int k) {
+  constexpr int CPT = SPT * (int)sizeof(T) / 16;
+  static_assert(CPT >= 1 && CPT <= 8, "a run is at most one 128-byte line");
+  return ((lane * CPT + ((lane / (8 / CPT)) & (CPT - 1))) * 16) ^ (k * 16);
+}
+// ... and of chunk lane + 32 * k of the warp's samples in order
+template <typename T, int SPT>
+__device__ __forceinline__ int warp1d_line(int lane, int k) {
+  constexpr int CPT = SPT * (int)sizeof(T) / 16;
+  const int base = ((lane & ~(CPT - 1)) + ((lane & (CPT - 1)) ^ ((lane / 8) & (CPT - 1)))) * 16;
+  return (CPT == 8 && (k & 1)) ? (base ^ 64) + k * 512 : base + k * 512;
+}
+
+__device__ __forceinline__ void warp1d_copy16(void* dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+}
+
+// Starts the copy of samples tw .. tw + 32 * SPT - 1 of a row of N samples (zeros outside) into the staging
+// buffer; complete after cp.async wait and __syncwarp.  up > 1: the row holds N / up values and sample t is
+// row[t / up] / up.
+template <typename T, int SPT>
+__device__ __forceinline__ void warp1d_fetch(const T* __restrict__ xr, int tw, int lane, int N, int up, unsigned char* st) {
+  constexpr int VEC = 16 / (int)sizeof(T), CPT = SPT / VEC;
+  if (up == 1 && (reinterpret_cast<uintptr_t>(xr) & 15) == 0) {   // warp-uniform
+    const T* p = xr + tw + lane * VEC;
+    if (tw >= 0 && tw + 32 * SPT <= N) {                          // the whole span is inside the signal
+#pragma unroll
+      for (int k = 0; k < CPT; ++k) async_copy16(st + warp1d_line<T, SPT>(lane, k), p + 32 * VEC * k);
+    } else {
+#pragma unroll
+      for (int k = 0; k < CPT; ++k) {
+        const int t = tw + (lane + 32 * k) * VEC;
+        const int n = (t >= 0 && t < N) ? imin(N - t, VEC) * (int)sizeof(T) : 0;      // bytes inside the signal
+        warp1d_copy16(st + warp1d_line<T, SPT>(lane, k), n ? p + 32 * VEC * k : xr, n);
+      }
+    }
+  } else {
+    const unsigned limit = (unsigned)(N / up * up);
+    const float inv = 1.f / (float)up;
+#pragma unroll 8                                                    // not whole: the loop appears twice and the code must fit the instruction cache
+    for (int k = 0; k < SPT; ++k) {
+      const int idx = lane + 32 * k;
+      const unsigned t = (unsigned)(tw + idx);                      // negative positions wrap beyond the limit
+      T* d = reinterpret_cast<T*>(st + warp1d_own<T, SPT>(idx / SPT, (idx / VEC) & (CPT - 1))) + (idx & (VEC - 1));
+      if (sizeof(T) == 4 && up == 1) {
+        async_copy4_zfill(d, t < limit ? xr + t : xr, t < limit);
+      } else {
+        float v = 0.f;
+        if (t < limit) v = up == 1 ? Elem<T>::to_f(xr[t]) : Elem<T>::to_f(xr[t / (unsigned)up]) * inv;
+        *d = Elem<T>::from_f(v);
+      }
+    }
+  }
+}
+
+// This thread's run
+template <typename T, int SPT>
+__device__ __forceinline__ void warp1d_read(const unsigned char* st, int lane, float (&v)[SPT]) {
+  constexpr int VEC = 16 / (int)sizeof(T), CPT = SPT / VEC;
+#pragma unroll
+  for (int k = 0; k < CPT; ++k) {
+    Chunk<T, 16> ch;
+    ch.raw = *reinterpret_cast<const uint4*>(st + warp1d_own<T, SPT>(lane, k));
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) v[k * VEC + i] = Elem<T>::to_f(ch.get(i));
+  }
+}
+
 // Levels J..L from the low band of level J-1 (`src`, 2*NJ values per thread); returns the
 // reconstruction R_{J-1} in `rec` (2*NJ values): conv(lo) + R_J and conv(hi), then synthesis.
 template <int K, int L, int J, int NJ>
@@ -107,122 +190,261 @@ struct Warp1dLevel {
 };
 #endif
 
-template <typename T, int K, int L>
-__global__ void __launch_bounds__(kWarp1dWarps * 32)
+// Dynamic shared memory: per warp two staging buffers and two tap-set buffers
+template <typename T, int K, int L, int SPT>
+constexpr size_t warp1d_smem_bytes() { return (size_t)kWarp1dWarps * 2 * (32 * SPT * sizeof(T) + warp1d_tap_words(K, L) * 16); }
+
+// A warp walks over (row, segment) items and copies the samples and taps of the next one while it computes
+// the current one.  Registers: the run, the accumulated output and one level's bands are live at once
+// (about four SPT values), which fits 64 registers (32 warps per SM) with 16 samples and 128 (16 warps)
+// with 32.
+template <typename T, int K, int L, int SPT>
+__global__ void __launch_bounds__(kWarp1dWarps * 32, SPT == 32 ? 2 : (K <= 5 && L <= 3 ? 4 : 3))
 wt1d_warp_kernel(const __grid_constant__ Warp1dArgs a) {
 #ifdef __CUDA_ARCH__
-  static_assert(L >= 0 && L <= kWarp1dMaxLevels && K <= 7, "levels beyond 2^L = 16 samples per thread take the CTA-tile kernel");
-  constexpr int SPT = kWarp1dSpt, R = K / 2;
-  constexpr int HL = (R * (1 << L) + SPT - 1) / SPT;   // neighbour-only lanes per side
-  constexpr int SEG = (32 - 2 * HL) * SPT;             // output samples per warp
+  static_assert(L >= 0 && L <= kWarp1dMaxLevels && (1 << L) <= SPT && K <= 7, "deeper cascades take the CTA-tile kernel");
+  constexpr int R = K / 2;
+  constexpr int HL = warp1d_halo(K, L, SPT);           // neighbour-only lanes per side
+  constexpr int SEG = warp1d_segment(K, L, SPT);       // output samples per warp
   constexpr int VEC = 16 / (int)sizeof(T);             // samples per 128-bit access
-  constexpr int NCH = SPT / VEC;                       // 128-bit accesses per thread
-  typedef typename RawChunk<16>::type raw_t;
-  constexpr int TS = (K + 1 + 3) / 4 * 4;              // floats per tap set
-  constexpr int NW4 = (1 + 2 * L) * TS / 4;            // 128-bit words of a channel's tap sets (<= 18)
-  __shared__ __align__(16) float stage[kWarp1dWarps][32 * kWarp1dPitch];
-  __shared__ __align__(16) float taps[kWarp1dWarps][NW4 * 4];
+  constexpr int CPT = SPT / VEC;                       // 128-bit accesses per thread
+  constexpr int NW4 = warp1d_tap_words(K, L);
+  constexpr int BUF = 32 * SPT * (int)sizeof(T), STEP = BUF + NW4 * 16;
+  extern __shared__ __align__(128) unsigned char warp1d_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float* st = stage[warp];
-  // (row, segment) of this warp; the launcher keeps the warp count below 2^31
-  const unsigned wid = blockIdx.x * (unsigned)kWarp1dWarps + warp;
-  if (wid >= (unsigned)a.nwarps) return;               // whole warps leave together
-  const unsigned row = wid / (unsigned)a.nseg;
-  const int seg = (int)(wid - row * (unsigned)a.nseg);
-  const unsigned n = row / (unsigned)a.C, c = row - n * (unsigned)a.C;
-  const T* xr = static_cast<const T*>(a.x) + n * a.xs0 + c * a.xs1;
-  T* yr = static_cast<T*>(a.y) + n * a.ys0 + c * a.ys1;
-  // tap sets of the row's channel: requested first, stored after the samples have been requested
-  float4 wq = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (lane < NW4) wq = __ldg(reinterpret_cast<const float4*>(a.packed + (size_t)c * a.wstride) + lane);
-  const float* wch = taps[warp];
-  const int tw = seg * SEG - HL * SPT;                 // first sample of the warp: a multiple of 16, negative in a row's first segment
-  const int t0 = tw + lane * SPT;                      // first sample of this thread
+  unsigned char* const buf0 = warp1d_smem + warp * 2 * STEP;
+  const unsigned nwarps = (unsigned)a.nwarps, stride = gridDim.x * (unsigned)kWarp1dWarps;   // the launcher keeps the sum below 2^32
+  struct Item { unsigned n, c; int tw; };
+  auto item = [&](unsigned wid) {
+    const unsigned row = wid / (unsigned)a.nseg;
+    Item it;
+    it.tw = (int)(wid - row * (unsigned)a.nseg) * SEG - HL * SPT;   // first sample: a multiple of SPT, negative in a row's first segment
+    it.n = row / (unsigned)a.C;
+    it.c = row - it.n * (unsigned)a.C;
+    return it;
+  };
+  auto fetch = [&](const Item& it, unsigned char* st) {
+    warp1d_fetch<T, SPT>(static_cast<const T*>(a.x) + it.n * a.xs0 + it.c * a.xs1, it.tw, lane, a.N, a.up, st);
+    if (lane < NW4) async_copy16(st + BUF + 16 * lane, a.packed + (size_t)it.c * a.wstride + 4 * lane);
+  };
+  unsigned wid = blockIdx.x * (unsigned)kWarp1dWarps + warp;
+  if (wid >= nwarps) return;                           // whole warps leave together
+  Item cur = item(wid);
+  fetch(cur, buf0);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int which = 0;; which ^= 1) {
+    unsigned char* st = buf0 + which * STEP;
+    wid += stride;
+    Item next = cur;
+    if (wid < nwarps) {
+      next = item(wid);
+      fetch(next, buf0 + (which ^ 1) * STEP);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+    float xv[SPT];
+    warp1d_read<T, SPT>(st, lane, xv);
+    const float* wch = reinterpret_cast<const float*>(st + BUF);
 
-  // ---- load: 16 samples, zeros outside the signal
-  float xv[SPT];
-  if ((reinterpret_cast<uintptr_t>(xr) & 15) == 0) {   // warp-uniform
+    // ---- levels, deepest first (recursion), then the base convolution and the bias
+    float out[SPT];
+    if constexpr (L >= 1) {
+      Warp1dLevel<K, L, 1, SPT / 2>::run(xv, wch, out);
+    } else {
 #pragma unroll
-    for (int v = 0; v < NCH; ++v) {
-      const int t = t0 + v * VEC;
-      if (t >= 0 && t + VEC <= a.N) {
+      for (int o = 0; o < SPT; ++o) out[o] = 0.f;
+    }
+    {
+      const float bias = wch[K];
+#pragma unroll
+      for (int o = 0; o < SPT; ++o) out[o] += bias;
+      float ext[SPT + 2 * R];
+      warp1d_extend<SPT, R>(xv, ext);
+      warp1d_conv<SPT, K>(ext, wch, out);
+    }
+
+    // ---- store (crop to the signal: wtconv1d.py:76); the neighbour-only lanes' samples are left out
+    T* yr = static_cast<T*>(a.y) + cur.n * a.ys0 + cur.c * a.ys1;
+    __syncwarp();                                      // everyone has read its run
+    if (a.pool > 1) {
+      // average of `pool` consecutive samples: a segment starts on a multiple of SPT samples, so the
+      // groups are local; the averages leave coalesced through the staging buffer
+      const int per = SPT / a.pool;
+      const float inv = 1.f / (float)a.pool;
+      T* sp = reinterpret_cast<T*>(st);
+#pragma unroll
+      for (int w = 1; w < 8; w *= 2)
+        if (w < a.pool) {
+#pragma unroll
+          for (int o = 0; o + w < SPT; o += 2 * w) out[o] += out[o + w];
+        }
+#pragma unroll
+      for (int o = 0; o < SPT; ++o)
+        if ((o & (a.pool - 1)) == 0) sp[lane * per + o / a.pool] = Elem<T>::from_f(out[o] * inv);
+      __syncwarp();
+      const int No = a.N / a.pool, o0 = cur.tw / a.pool;
+      for (int idx = HL * per + lane; idx < (32 - HL) * per; idx += 32)
+        if (o0 + idx < No) yr[o0 + idx] = sp[idx];
+    } else {
+#pragma unroll
+      for (int k = 0; k < CPT; ++k) {
         Chunk<T, 16> ch;
-        ch.raw = __ldg(reinterpret_cast<const raw_t*>(xr + t));
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) xv[v * VEC + i] = Elem<T>::to_f(ch.get(i));
-      } else {
-#pragma unroll
-        for (int i = 0; i < VEC; ++i) xv[v * VEC + i] = (t + i >= 0 && t + i < a.N) ? Elem<T>::to_f(xr[t + i]) : 0.f;
+        for (int i = 0; i < VEC; ++i) ch.set(i, Elem<T>::from_f(out[k * VEC + i]));
+        *reinterpret_cast<uint4*>(st + warp1d_own<T, SPT>(lane, k)) = ch.raw;
       }
-    }
-  } else {
-    // coalesced element-wise loads of the warp's 512 samples into the staging buffer, then each
-    // thread's run of 16 (runs are 20 floats apart: 128-bit reads without bank conflicts)
+      __syncwarp();
+      if ((reinterpret_cast<uintptr_t>(yr) & 15) == 0) {
+        T* p = yr + cur.tw + lane * VEC;
+        const bool whole = cur.tw + (32 - HL) * SPT <= a.N;
 #pragma unroll
-    for (int k = 0; k < SPT; ++k) {
-      const int idx = lane + 32 * k;
-      const int t = tw + idx;
-      st[idx + (idx >> 4) * 4] = (t >= 0 && t < a.N) ? Elem<T>::to_f(xr[t]) : 0.f;
-    }
-    __syncwarp();
+        for (int k = 0; k < CPT; ++k) {
+          const int q = lane + 32 * k, t = cur.tw + q * VEC;
+          if (q < HL * CPT || q >= (32 - HL) * CPT) continue;
+          const uint4 v = *reinterpret_cast<const uint4*>(st + warp1d_line<T, SPT>(lane, k));
+          if (whole || t + VEC <= a.N) *reinterpret_cast<uint4*>(p + 32 * VEC * k) = v;
+          else {
+            Chunk<T, 16> ch;
+            ch.raw = v;
 #pragma unroll
-    for (int v = 0; v < SPT / 4; ++v) {
-      const float4 q = *reinterpret_cast<const float4*>(st + lane * kWarp1dPitch + 4 * v);
-      xv[4 * v] = q.x; xv[4 * v + 1] = q.y; xv[4 * v + 2] = q.z; xv[4 * v + 3] = q.w;
-    }
-    __syncwarp();
-  }
-
-  if (lane < NW4) reinterpret_cast<float4*>(taps[warp])[lane] = wq;
-  __syncwarp();
-
-  // ---- levels, deepest first (recursion), then the base convolution and the bias
-  float out[SPT];
-  if constexpr (L >= 1) {
-    Warp1dLevel<K, L, 1, SPT / 2>::run(xv, wch, out);
-  } else {
-#pragma unroll
-    for (int o = 0; o < SPT; ++o) out[o] = 0.f;
-  }
-  {
-    const float bias = wch[K];
-#pragma unroll
-    for (int o = 0; o < SPT; ++o) out[o] += bias;
-    float ext[SPT + 2 * R];
-    warp1d_extend<SPT, R>(xv, ext);
-    warp1d_conv<SPT, K>(ext, wch, out);
-  }
-
-  // ---- store (crop to the signal: wtconv1d.py:76); the neighbour-only lanes store nothing
-  const bool owner = lane >= HL && lane < 32 - HL;
-  if ((reinterpret_cast<uintptr_t>(yr) & 15) == 0) {
-    if (owner) {
-#pragma unroll
-      for (int v = 0; v < NCH; ++v) {
-        const int t = t0 + v * VEC;
-        if (t + VEC <= a.N) {
-          Chunk<T, 16> ch;
-#pragma unroll
-          for (int i = 0; i < VEC; ++i) ch.set(i, Elem<T>::from_f(out[v * VEC + i]));
-          *reinterpret_cast<raw_t*>(yr + t) = ch.raw;
-        } else {
-#pragma unroll
-          for (int i = 0; i < VEC; ++i)
-            if (t + i < a.N) yr[t + i] = Elem<T>::from_f(out[v * VEC + i]);
+            for (int i = 0; i < VEC; ++i)
+              if (t + i < a.N) yr[t + i] = ch.get(i);
+          }
+        }
+      } else {
+#pragma unroll 8
+        for (int k = 0; k < SPT; ++k) {
+          const int idx = lane + 32 * k, t = cur.tw + idx;
+          if (idx >= HL * SPT && idx < (32 - HL) * SPT && t < a.N)
+            yr[t] = *(reinterpret_cast<const T*>(st + warp1d_own<T, SPT>(idx / SPT, (idx / VEC) & (CPT - 1))) + (idx & (VEC - 1)));
         }
       }
     }
-  } else {
+    if (wid >= nwarps) break;
+    cur = next;
+    __syncwarp();                                      // the buffer is refilled in the next iteration
+  }
+#endif
+}
+
+// ---------------------------------------------------------------------------
+// Parameter gradients: with S = un-normalised sub-bands of x (level 0: x itself) and G the same of
+// the output gradient, every gradient of a channel follows from the K-tap correlation sums
+//     stat[set][k] = sum over samples and positions p of G_set[p] * S_set[p + k - K/2]
+// (see wt2d_wgrad.cuh).  A warp owns one channel and walks over (sample, segment) items: both
+// cascades stay in registers, and so do all (1 + 2L) * K + 1 sums until the walk ends; then the lanes
+// meet by shuffles, the warps of a CTA in shared memory and the CTAs of a channel in `stats` (fp32
+// atomics, a few CTAs per channel).  One pass over x and g with no intermediate in memory.
+// ---------------------------------------------------------------------------
+struct Wgrad1dArgs {
+  const void* x;
+  const void* g;
+  float* stats;           // (1 + 4L, K*K + 1, C) as the one-row image of the 2-D kernels lays them out, zeroed
+  int B, C, N;
+  int up;                 // output stride: g holds N / up samples (see Warp1dArgs)
+  int nseg, nsplit;       // segments per row, CTAs per channel
+  long long items;        // B * nseg
+  long long xs0, xs1, gs0, gs1;
+};
+
+#ifdef __CUDA_ARCH__
+template <int NJ, int K, int NA>
+__device__ __forceinline__ void warp1d_correlate(const float (&s)[NJ], const float (&g)[NJ], float (&acc)[NA], int at) {
+  constexpr int R = K / 2;
+  float ext[NJ + 2 * R];
+  warp1d_extend<NJ, R>(s, ext);
 #pragma unroll
-    for (int v = 0; v < SPT / 4; ++v)
-      *reinterpret_cast<float4*>(st + lane * kWarp1dPitch + 4 * v) = make_float4(out[4 * v], out[4 * v + 1], out[4 * v + 2], out[4 * v + 3]);
-    __syncwarp();
+  for (int k = 0; k < K; ++k)
 #pragma unroll
-    for (int k = 0; k < SPT; ++k) {
-      const int idx = lane + 32 * k;
-      const int t = tw + idx;
-      if (idx >= HL * SPT && idx < (32 - HL) * SPT && t < a.N) yr[t] = Elem<T>::from_f(st[idx + (idx >> 4) * 4]);
+    for (int o = 0; o < NJ; ++o) acc[at + k] = fmaf(g[o], ext[o + k], acc[at + k]);
+}
+
+template <int K, int L, int J, int NJ, int NA>
+struct Warp1dGradLevel {
+  static __device__ __forceinline__ void run(const float (&x)[2 * NJ], const float (&g)[2 * NJ], float (&acc)[NA]) {
+    float xs[NJ], gs[NJ];
+#pragma unroll
+    for (int o = 0; o < NJ; ++o) { xs[o] = x[2 * o] - x[2 * o + 1]; gs[o] = g[2 * o] - g[2 * o + 1]; }
+    warp1d_correlate<NJ, K, NA>(xs, gs, acc, K + 1 + (2 * (J - 1) + 1) * K);
+#pragma unroll
+    for (int o = 0; o < NJ; ++o) { xs[o] = x[2 * o] + x[2 * o + 1]; gs[o] = g[2 * o] + g[2 * o + 1]; }
+    warp1d_correlate<NJ, K, NA>(xs, gs, acc, K + 1 + 2 * (J - 1) * K);
+    if constexpr (J < L) Warp1dGradLevel<K, L, J + 1, NJ / 2, NA>::run(xs, gs, acc);
+  }
+};
+#endif
+
+// Dynamic shared memory: two buffers of the x run and the g run per warp (the next item is copied while
+// this one is computed)
+template <typename T, int SPT>
+constexpr size_t warp1d_wgrad_smem() { return (size_t)kWarp1dWarps * 4 * 32 * SPT * sizeof(T); }
+
+template <typename T, int K, int L, int SPT>
+__global__ void __launch_bounds__(kWarp1dWarps * 32, (K <= 5 && L <= 4) ? 2 : 1)
+wt1d_wgrad_kernel(const __grid_constant__ Wgrad1dArgs a) {
+#ifdef __CUDA_ARCH__
+  constexpr int HL = warp1d_halo(K, L, SPT), SEG = warp1d_segment(K, L, SPT);
+  constexpr int NA = K + 1 + 2 * L * K;                // base taps, sum of g, then (low, high) taps per level
+  constexpr int BUF = 32 * SPT * (int)sizeof(T);
+  extern __shared__ __align__(128) unsigned char warp1d_smem[];
+  static_assert(NA * (int)sizeof(float) <= 4 * BUF, "the sums of a warp fit its buffers");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned char* st = warp1d_smem + warp * 4 * BUF;
+  const int c = (int)(blockIdx.x / (unsigned)a.nsplit), split = (int)(blockIdx.x - (unsigned)c * (unsigned)a.nsplit);
+  const bool owner = lane >= HL && lane < 32 - HL;
+  float acc[NA];
+#pragma unroll
+  for (int k = 0; k < NA; ++k) acc[k] = 0.f;
+  const long long step = (long long)a.nsplit * kWarp1dWarps;
+  auto fetch = [&](long long it, unsigned char* buf) {
+    if (it < a.items) {
+      const int n = (int)(it / a.nseg), seg = (int)(it - (long long)n * a.nseg);
+      const int tw = seg * SEG - HL * SPT;
+      warp1d_fetch<T, SPT>(static_cast<const T*>(a.x) + n * a.xs0 + c * a.xs1, tw, lane, a.N, 1, buf);
+      warp1d_fetch<T, SPT>(static_cast<const T*>(a.g) + n * a.gs0 + c * a.gs1, tw, lane, a.N, a.up, buf + BUF);
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  long long it = (long long)split * kWarp1dWarps + warp;
+  fetch(it, st);
+  for (int cur = 0; it < a.items; it += step, cur ^= 1) {
+    fetch(it + step, st + (cur ^ 1) * 2 * BUF);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+    float xv[SPT], gv[SPT];
+    warp1d_read<T, SPT>(st + cur * 2 * BUF, lane, xv);
+    warp1d_read<T, SPT>(st + cur * 2 * BUF + BUF, lane, gv);
+#pragma unroll
+    for (int o = 0; o < SPT; ++o) {                    // the outer lanes' positions belong to the neighbouring segments
+      gv[o] = owner ? gv[o] : 0.f;
+      acc[K] += gv[o];
+    }
+    warp1d_correlate<SPT, K, NA>(xv, gv, acc, 0);
+    if constexpr (L >= 1) Warp1dGradLevel<K, L, 1, SPT / 2, NA>::run(xv, gv, acc);
+    __syncwarp();                                      // the buffer is refilled in the next iteration
+  }
+#pragma unroll
+  for (int k = 0; k < NA; ++k) {
+    float v = acc[k];
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
+    if (lane == 0) reinterpret_cast<float*>(st)[k] = v;
+  }
+  __syncthreads();
+  constexpr int KK1 = K * K + 1, MID = (K / 2) * K;    // the K taps are the middle row of a K x K set
+  for (int e = threadIdx.x; e < NA; e += kWarp1dWarps * 32) {
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarp1dWarps; ++w) v += reinterpret_cast<const float*>(warp1d_smem + w * 4 * BUF)[e];
+    int slot;
+    if (e < K) slot = MID + e;
+    else if (e == K) slot = K * K;
+    else {
+      const int band = (e - K - 1) / K, k = (e - K - 1) - band * K;   // band = 2 * level + (0 low, 1 high)
+      slot = (1 + 4 * (band >> 1) + 2 * (band & 1)) * KK1 + MID + k;
+    }
+    atomicAdd(a.stats + (size_t)slot * a.C + c, v);
   }
 #endif
 }
@@ -230,9 +452,14 @@ wt1d_warp_kernel(const __grid_constant__ Warp1dArgs a) {
 // x, y: (B, C, N) with unit time stride; dtype 0 fp32, 1 bf16, 2 fp16.  Returns cudaErrorNotSupported
 // for combinations this kernel does not cover (the caller then takes the CTA-tile kernel).
 cudaError_t launch_wt1d_warp(const Warp1dArgs& a, int K, int L, int dtype, cudaStream_t stream);
+cudaError_t launch_wt1d_wgrad(const Wgrad1dArgs& a, int K, int L, int dtype, cudaStream_t stream);
+inline bool wt1d_warp_levels(int K, int L) {
+  return L >= 0 && L <= kWarp1dMaxLevels && (K == 1 || K == 3 || K == 5 || K == 7);
+}
+// The pooled runs of a thread must be whole: strides that divide its 16 samples, up to eight of them
 inline bool wt1d_warp_supported(int K, int L, int stride, long long x_tstride, long long y_tstride) {
-  return stride == 1 && L >= 0 && L <= kWarp1dMaxLevels && (K == 1 || K == 3 || K == 5 || K == 7) &&
-         x_tstride == 1 && y_tstride == 1;
+  return (stride == 1 || stride == 2 || stride == 4 || stride == 8) && wt1d_warp_levels(K, L) && x_tstride == 1 &&
+         y_tstride == 1;
 }
 
 }  // namespace wt

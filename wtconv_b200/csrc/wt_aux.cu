@@ -43,7 +43,7 @@ __global__ void param_grads_kernel(GradArgs a) {
 cudaError_t launch_param_grads(const GradArgs& a, int param_dtype, cudaStream_t stream) {
   const int nsub = (a.ndim == 2) ? 4 : 2;
   const long long total = (long long)(1 + nsub * a.L) * a.C;
-  const int threads = 128;
+  const int threads = 64;
   const int blocks = (int)((total + threads - 1) / threads);
   switch (param_dtype) {
     case 0: param_grads_kernel<float><<<blocks, threads, 0, stream>>>(a); break;

@@ -107,6 +107,31 @@ struct GradArgs {
   double gain[kMaxLevels];       // (analysis tap * synthesis tap)^(level+1)
 };
 
+// The taps of one set: gw[t] = factor * sums[t], returns <w, sums>.  The loads of eight taps are issued
+// together: the kernel is one thread per (set, channel), a few thousand in all, and lasts as long as its
+// chain of dependent loads (25 taps one after the other: 20 us; in four batches: 5 us).
+template <typename P>
+WT_HD float param_grad_taps(const float* sums, int step, const P* w, P* gw, int taps, float factor) {
+  constexpr int U = 8;
+  float dot = 0.f;
+  for (int t0 = 0; t0 < taps; t0 += U) {
+    float corr[U], wv[U];
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+      const int t = imin(t0 + i, taps - 1);
+      corr[i] = sums[(size_t)t * step];
+      wv[i] = Elem<P>::to_f(w[t]);
+    }
+#pragma unroll
+    for (int i = 0; i < U; ++i)
+      if (t0 + i < taps) {
+        gw[t0 + i] = Elem<P>::from_f(factor * corr[i]);
+        dot = fmaf(wv[i], corr[i], dot);
+      }
+  }
+  return dot;
+}
+
 template <typename P>
 WT_HD void param_grad_item(const GradArgs& a, long long idx) {
   const int nsub = (a.ndim == 2) ? 4 : 2;
@@ -120,12 +145,7 @@ WT_HD void param_grad_item(const GradArgs& a, long long idx) {
     const float sc = Elem<P>::to_f(static_cast<const P*>(a.base_scale)[c]);
     const P* w = static_cast<const P*>(a.base_w) + (size_t)c * taps;
     P* gw = static_cast<P*>(a.g_base_w) + (size_t)c * taps;
-    float dot = 0.f;
-    for (int t = 0; t < taps; ++t) {
-      const float corr = st[(size_t)(tap0 + t) * a.C];
-      gw[t] = Elem<P>::from_f(sc * corr);
-      dot = fmaf(Elem<P>::to_f(w[t]), corr, dot);
-    }
+    float dot = param_grad_taps<P>(st + (size_t)tap0 * a.C, a.C, w, gw, taps, sc);
     const float sum_g = st[(size_t)(a.K * a.K) * a.C];
     if (a.base_b) {
       static_cast<P*>(a.g_base_b)[c] = Elem<P>::from_f(sc * sum_g);
@@ -141,12 +161,7 @@ WT_HD void param_grad_item(const GradArgs& a, long long idx) {
     const float sc = Elem<P>::to_f(static_cast<const P*>(a.wavelet_scale[l])[oc]);
     const P* w = static_cast<const P*>(a.wavelet_w[l]) + (size_t)oc * taps;
     P* gw = static_cast<P*>(a.g_wavelet_w[l]) + (size_t)oc * taps;
-    float dot = 0.f;
-    for (int t = 0; t < taps; ++t) {
-      const float corr = st[(size_t)(tap0 + t) * a.C];
-      gw[t] = Elem<P>::from_f(sc * g * corr);
-      dot = fmaf(Elem<P>::to_f(w[t]), corr, dot);
-    }
+    const float dot = param_grad_taps<P>(st + (size_t)tap0 * a.C, a.C, w, gw, taps, sc * g);
     static_cast<P*>(a.g_wavelet_scale[l])[oc] = Elem<P>::from_f(g * dot);
   }
 }
