@@ -337,13 +337,15 @@ int wtconv2d_workspace_bytes(int B, int C, int H, int W, int K, int L, int dtype
   if (!bytes) return WTCONV_ERR_BAD_ARG;
   Layer2d ly;
   // The stage chain depends on the strides and on whether the base addresses are 16-byte aligned
-  // (the tensor maps of the channels-last kernels need that).  The size reported is the larger of
-  // both cases, so it holds for any pair of pointers with these strides.
+  // (the tensor maps of the channels-last kernels need that), and strided outputs take a chain of their
+  // own.  The size reported is the largest of these cases, so it holds for any pair of pointers with these
+  // strides and any output stride.
   const int st = make_layer2d(ly, nullptr, nullptr, B, C, H, W, K, L, 1, dtype, x_strides, y_strides);
   if (st) return st;
   long long floats = 0;
-  for (int variant = 0; variant < 2; ++variant) {
-    ly.x_align = ly.y_align = variant ? ly.elem_size : 16;
+  for (int variant = 0; variant < 4; ++variant) {
+    ly.x_align = ly.y_align = (variant & 1) ? ly.elem_size : 16;
+    ly.stride = (variant & 2) ? 2 : 1;
     const std::shared_ptr<const Chain2d> chp = cached_chain(ly);
     if (chp->status) return chp->status;
     if (chp->scratch_floats > floats) floats = chp->scratch_floats;
@@ -434,6 +436,12 @@ int wtconv2d_forward(const void* x, void* y, const float* packed, void* workspac
                                    sg.rin_off < 0 ? nullptr : static_cast<void*>(ws + sg.rin_off), cs);
         break;
       }
+      case 7:
+        e = launch_planar(sg.planar, in_dtype, xin, final_stage ? y : static_cast<void*>(rout), rin, packed, cs);
+        break;
+      case 8:
+        e = launch_planar_lowpass(sg.low, in_dtype, xin, ws, cs);
+        break;
       default:
         e = launch_wt2d(sg.plan, in_dtype, xin, final_stage ? y : nullptr, packed, rin, rout, (size_t)sg.smem_bytes, cs);
         break;

@@ -331,23 +331,27 @@ void grad_stats(const LayerDesc& d, const Tensor& x, const Tensor& g, Tensor& st
 variable_list param_grads(const LayerDesc& d, const Tensor& stats) {
   const int L = d.L;
   cudaStream_t stream = c10::cuda::getCurrentCUDAStream(stats.device().index()).stream();
-  std::vector<Tensor> hold;
-  variable_list grads;
-  for (const Tensor& p : d.params) {
-    hold.push_back(p.defined() ? p.detach().contiguous() : Tensor());
-    grads.push_back(p.defined() ? at::empty_like(hold.back(), at::MemoryFormat::Contiguous) : Tensor());
+  variable_list grads(d.params.size());
+  std::vector<Tensor> copies;                       // of parameters that are not contiguous
+  std::vector<const void*> p(d.params.size(), nullptr);
+  std::vector<void*> g(d.params.size(), nullptr);
+  for (size_t i = 0; i < d.params.size(); ++i) {
+    const Tensor& t = d.params[i];
+    if (!t.defined()) continue;
+    if (t.is_contiguous()) p[i] = t.const_data_ptr();
+    else { copies.push_back(t.detach().contiguous()); p[i] = copies.back().const_data_ptr(); }
+    grads[i] = at::detail::empty_cuda(t.sizes(), t.scalar_type(), t.device(), std::nullopt);
+    g[i] = grads[i].data_ptr();
   }
   const double tap = tap_magnitude(d.ndim, d.filter_dtype);
   std::vector<const void*> ww(std::max(L, 1)), ws(std::max(L, 1));
   std::vector<void*> gw(std::max(L, 1)), gsc(std::max(L, 1));
   for (int i = 0; i < L; ++i) {
-    ww[i] = hold[3 + 2 * i].const_data_ptr(); ws[i] = hold[4 + 2 * i].const_data_ptr();
-    gw[i] = grads[3 + 2 * i].data_ptr(); gsc[i] = grads[4 + 2 * i].data_ptr();
+    ww[i] = p[3 + 2 * i]; ws[i] = p[4 + 2 * i];
+    gw[i] = g[3 + 2 * i]; gsc[i] = g[4 + 2 * i];
   }
-  check(wtconv_param_grads(d.ndim, d.C, d.K, L, dtype_code(hold[0].scalar_type()), tap, tap, stats.const_data_ptr<float>(),
-                           hold[0].const_data_ptr(), hold[1].defined() ? hold[1].const_data_ptr() : nullptr,
-                           hold[2].const_data_ptr(), ww.data(), ws.data(), grads[0].data_ptr(),
-                           grads[1].defined() ? grads[1].data_ptr() : nullptr, grads[2].data_ptr(), gw.data(), gsc.data(), stream),
+  check(wtconv_param_grads(d.ndim, d.C, d.K, L, dtype_code(d.params[0].scalar_type()), tap, tap, stats.const_data_ptr<float>(),
+                           p[0], p[1], p[2], ww.data(), ws.data(), g[0], g[1], g[2], gw.data(), gsc.data(), stream),
         "wtconv_param_grads");
   return grads;
 }

@@ -8,6 +8,7 @@
 
 #include "wt2d_cl_host.h"
 #include "wt2d_plan.h"
+#include "wt2d_planar_host.h"
 #include "wt2d_quad.cuh"
 #include "wt2d_regplane.cuh"
 
@@ -219,8 +220,11 @@ struct Stage2d {
   // 2: four-warp 14 x 14 level kernel (quad), 3: channels-last level stage (cl),
   // 4: channels-last deep stage (deep), 5: channels-last sub-band pyramid, 6: channels-last low-pass
   // planes (5 and 6 read the layer input or a low-pass plane set of cl.H x cl.W; 6 writes one
-  // level down to rout_off and, if rin_off >= 0, two levels down there)
+  // level down to rout_off and, if rin_off >= 0, two levels down there), 7: planar kernel (planar),
+  // 8: low-pass planes of the planar chain (low; reads xin_off, writes at its own offsets)
   int kind = 0;
+  PlanarStage planar;
+  PlanarLowpass low;
   RegPlane reg;
   QuadPlane quad;
   ClStage cl;
@@ -424,6 +428,174 @@ inline void plan_cl_level(ClStage& s, const Layer2d& ly, int level, int H, int W
   }
 }
 
+// Widest access (4, 2 or 1 elements of a row) that strides and base alignment allow
+inline int row_vec(const long long* s, int elem_size, int align) {
+  for (int v = 4; v >= 2; v /= 2)
+    if (s[3] == 1 && align >= imin(16, v * elem_size) && s[0] % v == 0 && s[1] % v == 0 && s[2] % v == 0) return v;
+  return 1;
+}
+
+// One planar stage (wt2d_planar.cuh) on the plane of level `first`: levels first+1 .. first+nlev.  `x_src`:
+// the stage reads the layer input (first 0: directly, first 1: as 2 x 2 sums), else an fp32 plane set in
+// scratch.  Returns false when no channel group fits.
+inline bool plan_planar(PlanarStage& p, const Layer2d& ly, const int* Hl, const int* Wl, int first, int nlev, bool final_stage,
+                        bool tiled, bool x_src, bool cl) {
+  p = PlanarStage();
+  p.B = ly.B; p.C = ly.C; p.K = ly.K; p.nlev = nlev; p.lvl0 = first;
+  p.has_base = final_stage ? 1 : 0;
+  p.tiled = tiled ? 1 : 0;
+  for (int j = 0; j <= nlev; ++j) { p.h[j] = Hl[first + j]; p.w[j] = Wl[first + j]; }
+  const int h1 = cdiv(p.h[0], 2), w1 = cdiv(p.w[0], 2);
+  if (nlev == 0) { p.h[1] = h1; p.w[1] = w1; }
+  p.wstride = packed_channel_floats(ly.K, 2, ly.L);
+  p.shift = (x_src && first == 1) ? 1 : 0;
+  p.Hsrc = p.shift ? ly.H : p.h[0];
+  p.Wsrc = p.shift ? ly.W : p.w[0];
+  auto dense = [&](int h, int w, long long* s) {
+    s[0] = (long long)ly.C * h * w;
+    if (cl) { s[1] = 1; s[2] = (long long)w * ly.C; s[3] = ly.C; }
+    else { s[1] = (long long)h * w; s[2] = w; s[3] = 1; }
+  };
+  if (x_src) { for (int i = 0; i < 4; ++i) p.xs[i] = ly.xs[i]; }
+  else dense(p.h[0], p.w[0], p.xs);
+  if (final_stage) { for (int i = 0; i < 4; ++i) p.ys[i] = ly.ys[i]; }
+  else dense(p.h[0], p.w[0], p.ys);
+  dense(h1, w1, p.rs);
+  p.out_stride = final_stage ? ly.stride : 1;
+  p.Ho = cdiv(p.h[0], p.out_stride); p.Wo = cdiv(p.w[0], p.out_stride);
+  const int xe = x_src ? ly.elem_size : 4, xa = x_src ? ly.x_align : 16;
+  p.xvec = row_vec(p.xs, xe, xa);
+  p.yvec = final_stage ? row_vec(p.ys, ly.elem_size, ly.y_align) : row_vec(p.ys, 4, 16);
+  p.rvec = row_vec(p.rs, 4, 16) >= 2 ? 1 : 0;
+  // channel chunk of a channels-last source: 16, 8 or 4 bytes
+  auto chunk = [&](int G) {
+    if (!cl) return 0;
+    for (int bytes = 16; bytes >= 4; bytes /= 2) {
+      const int v = bytes / xe;
+      if (v <= G && xa >= bytes && p.xs[1] == 1 && p.xs[0] % v == 0 && p.xs[2] % v == 0 && p.xs[3] % v == 0) return v;
+    }
+    return 0;
+  };
+  auto geometry = [&](int G) {
+    p.G = G;
+    if (!tiled) {
+      p.TH = round_up(h1, 4); p.TW = round_up(w1, 4);
+    } else if (cl && G >= 8) {          // eight channels: 16 x 16 positions keep two CTAs on an SM
+      p.TH = round_up(cdiv(h1, cdiv(h1, 16)), 4); p.TW = round_up(cdiv(w1, cdiv(w1, 16)), 4);
+    } else {
+      const int th = G >= 4 ? 16 : 32;
+      p.TH = round_up(cdiv(h1, cdiv(h1, th)), 4); p.TW = round_up(cdiv(w1, cdiv(w1, 32)), 4);
+    }
+    p.xchunk = chunk(G);
+    return planar_layout(p);
+  };
+  // Channel group: the one that keeps most warps busy (planar_layout) with two CTAs on an SM, failing that
+  // with one; wider groups win a near tie (fewer barriers per plane).  A channels-last source read in
+  // chunks of less than 16 bytes wastes more of every sector, element by element most.
+  int pick = 0;
+  for (int limit = kSmemTwoPerSm; !pick; limit = kSmemLimitBytes) {
+    double best = 0.0;
+    for (int G = tiled && !cl ? 2 : 32; G >= 1; G /= 2) {
+      if (G > 1 && G / 2 >= ly.C) continue;
+      if (geometry(G) > limit) continue;
+      double score = p.score;
+      if (cl) score *= p.xchunk * xe >= 16 ? 1.0 : p.xchunk * xe == 8 ? 0.8 : p.xchunk ? 0.5 : 0.3;
+      // with less than two CTAs per SM, the smaller group of a near tie spreads over more SMs
+      if (score > best * (p.total < 2 * 148 ? 0.97 : 1.03)) { best = score; pick = G; }
+    }
+    if (limit == kSmemLimitBytes) break;
+  }
+  if (!pick) return false;
+  geometry(pick);
+  if (p.total >= (1LL << 31) - 65536 || p.nlev > kPlanarMaxLev) return false;
+  planar_grid(p);
+  return true;
+}
+
+// Launch chain of the planar kernels: whole planes of level q with every deeper level on chip, halo tiles of
+// one level above it.  q is the first level whose planes fit; the planes of level 1 are never stored (their
+// readers form them from the layer input), coarser ones come from one low-pass pass over the input.
+inline bool plan_planar_chain(Chain2d& ch, const Layer2d& ly, const std::vector<int>& Hl, const std::vector<int>& Wl) {
+  const bool cl = ly.xs[1] == 1 && ly.C > 1;
+  PlanarStage whole;
+  int q = 0;
+  for (; q < ly.L; ++q) {
+    if (Hl[q] > 128 || Wl[q] > 128) continue;
+    if (ly.L - q > kPlanarMaxLev) continue;
+    if (plan_planar(whole, ly, Hl.data(), Wl.data(), q, ly.L - q, q == 0, false, q <= 1, cl)) {
+      // planes that leave few warps on an SM lose more to idle issue slots than a tiled split costs (the top
+      // level's tiles are independent of the plane's size)
+      if (whole.smem_bytes <= kSmemTwoPerSm || whole.total < 148) break;
+    }
+  }
+  auto align4 = [](long long v) { return (v + 3) / 4 * 4; };
+  auto plane = [&](int j) { return align4((long long)ly.B * ly.C * Hl[j] * Wl[j]); };
+  const bool has_whole = q < ly.L;
+  std::vector<Stage2d> stages;
+  // scratch: R_2 (and deeper, alternating ends are not needed: they are small) first; R_1, the largest, shares
+  // its space with the planes that are dead when it is written
+  std::vector<long long> roff(q + 1, -1), poff(q + 1, -1);
+  long long base = 0, dead = 0;
+  if (q >= 2) { roff[2] = 0; base = plane(2); }
+  for (int j = 3; j <= q; ++j) { roff[j] = base + dead; dead += plane(j); }
+  const int top_low = has_whole ? q : q - 1;              // coarsest low-pass plane read
+  for (int j = 2; j <= top_low; ++j) { poff[j] = base + dead; dead += plane(j); }
+  long long r1 = 0;
+  const bool r1_used = (q >= 1 && has_whole) || q >= 2;
+  if (r1_used) { roff[1] = base; r1 = plane(1); }
+  if (q == 2 && has_whole) {                              // R_2's producer reads P_2 and its consumer writes R_1: no overlap with R_1's readers
+    // P_2 is dead once R_2 exists; R_2 itself lies below `base`
+  }
+  ch.scratch_floats = base + (dead > r1 ? dead : r1);
+  for (int j = 2; j <= top_low;) {                        // up to three levels per pass
+    Stage2d st;
+    st.kind = 8;
+    PlanarLowpass& lp = st.low;
+    const int from = j == 2 ? 0 : j - 1;
+    lp.B = ly.B; lp.C = ly.C; lp.H = Hl[from]; lp.W = Wl[from]; lp.cl = cl ? 1 : 0;
+    if (from == 0) { for (int i = 0; i < 4; ++i) lp.xs[i] = ly.xs[i]; }
+    else {
+      const long long hw = (long long)Hl[from] * Wl[from];
+      lp.xs[0] = ly.C * hw;
+      if (cl) { lp.xs[1] = 1; lp.xs[2] = (long long)Wl[from] * ly.C; lp.xs[3] = ly.C; }
+      else { lp.xs[1] = hw; lp.xs[2] = Wl[from]; lp.xs[3] = 1; }
+    }
+    for (int k = 0; k < 3; ++k) {
+      const int lev = from + 1 + k;
+      lp.off[k] = (lev >= j && lev <= top_low) ? poff[lev] : -1;
+    }
+    st.xin_off = from == 0 ? -1 : poff[from];
+    st.rin_off = -1; st.rout_off = 0; st.smem_bytes = 0;
+    stages.push_back(st);
+    j = from + 4;
+  }
+  if (has_whole) {
+    Stage2d st;
+    st.kind = 7;
+    st.planar = whole;
+    st.xin_off = q <= 1 ? -1 : poff[q];
+    st.rin_off = -1;
+    st.rout_off = q == 0 ? -1 : roff[q];
+    st.smem_bytes = whole.smem_bytes;
+    stages.push_back(st);
+  }
+  if (q > 0 || ly.L == 0) {
+    for (int j = q > 0 ? q : 1; j >= 1; --j) {
+      Stage2d st;
+      st.kind = 7;
+      const bool rin = ly.L > 0 && (j < q || has_whole);
+      if (!plan_planar(st.planar, ly, Hl.data(), Wl.data(), j - 1, ly.L == 0 ? 0 : 1, j == 1, true, j <= 2, cl)) return false;
+      st.xin_off = j <= 2 ? -1 : poff[j - 1];
+      st.rin_off = rin ? roff[j] : -1;
+      st.rout_off = j == 1 ? -1 : roff[j - 1];
+      st.smem_bytes = st.planar.smem_bytes;
+      stages.push_back(st);
+    }
+  }
+  ch.stages = stages;
+  return true;
+}
+
 // Builds the launch chain of one layer.
 inline Chain2d plan_layer(const Layer2d& ly, const Tuning2d& tune = Tuning2d()) {
   Chain2d ch;
@@ -521,12 +693,22 @@ inline Chain2d plan_layer(const Layer2d& ly, const Tuning2d& tune = Tuning2d()) 
       return ch;
     }
   }
+  // Kernel sizes 3, 5, 7 on every other tensor: the planar kernels.  (Channels-last tensors with K = 5 and
+  // stride 1 that the kernels above do not take keep the register-level chain below.)
+  const bool cl_tensor = ly.xs[1] == 1 && ly.ys[1] == 1 && ly.C > 1;
+  // A 7 x 7 plane fits a thread's registers whatever the layout (its loads then take a lane per plane, which
+  // the caches absorb): in shared memory its frames and tap sets leave a quarter of the warps resident.
+  const bool reg_whole = tune.cl >= 0 && !cl_tensor && ly.stride == 1 && ly.L >= 1 && regplane_supported(ly.K, ly.H, ly.W, ly.L);
+  if (tune.cl >= 0 && !reg_whole && (ly.K == 3 || ly.K == 7 || (ly.K == 5 && !(cl_tensor && ly.stride == 1)))) {
+    if (plan_planar_chain(ch, ly, Hl, Wl)) return ch;
+    ch = Chain2d();
+  }
   int qreg = -1;
   const bool untuned = !tune.force_tiled && !tune.tile_y && !tune.tile_x && !tune.tile_levels && !tune.group;
-  if ((untuned || tune.regplane > 0) && tune.regplane >= 0 && ly.xs[1] == 1 && ly.C > 1) {
+  if ((untuned || tune.regplane > 0) && tune.regplane >= 0 && ((ly.xs[1] == 1 && ly.C > 1) || reg_whole)) {
     for (int q = 0; q < ly.L; ++q) {
       if (!regplane_supported(ly.K, Hl[q], Wl[q], ly.L - q)) continue;
-      if (q == 0 && (ly.stride != 1 || ly.ys[1] != 1)) continue;
+      if (q == 0 && !reg_whole && (ly.stride != 1 || ly.ys[1] != 1)) continue;
       qreg = q;
       break;
     }

@@ -1,0 +1,59 @@
+// Launchers of the planar kernels: every compiled (type, kernel size) combination.
+#include "wt2d_planar.cuh"
+
+namespace wt {
+
+namespace {
+
+template <typename T, typename TO, int K, bool FINAL>
+cudaError_t launch_one(const PlanarStage& p, const void* x, void* out, const float* rin, const float* packed, cudaStream_t stream) {
+  auto kern = wt2d_planar_kernel<T, TO, K, FINAL>;
+  static bool done[kMaxDevices] = {false};
+  const cudaError_t e = allow_full_smem(kern, done);
+  if (e != cudaSuccess) return e;
+  kern<<<p.grid, p.nthreads, (size_t)p.smem_bytes, stream>>>(p, static_cast<const T*>(x), static_cast<TO*>(out), rin, packed);
+  return cudaGetLastError();
+}
+
+template <int K>
+cudaError_t launch_k(const PlanarStage& p, int dtype, const void* x, void* out, const float* rin, const float* packed, cudaStream_t st) {
+  if (!p.has_base) {
+    switch (dtype) {
+      case 0: return launch_one<float, float, K, false>(p, x, out, rin, packed, st);
+      case 1: return launch_one<__nv_bfloat16, float, K, false>(p, x, out, rin, packed, st);
+      default: return launch_one<__half, float, K, false>(p, x, out, rin, packed, st);
+    }
+  }
+  switch (dtype) {
+    case 0: return launch_one<float, float, K, true>(p, x, out, rin, packed, st);
+    case 1: return launch_one<__nv_bfloat16, __nv_bfloat16, K, true>(p, x, out, rin, packed, st);
+    default: return launch_one<__half, __half, K, true>(p, x, out, rin, packed, st);
+  }
+}
+
+}  // namespace
+
+cudaError_t launch_planar(const PlanarStage& p, int in_dtype, const void* x, void* out, const float* rin, const float* packed,
+                          cudaStream_t stream) {
+  switch (p.K) {
+    case 3: return launch_k<3>(p, in_dtype, x, out, rin, packed, stream);
+    case 5: return launch_k<5>(p, in_dtype, x, out, rin, packed, stream);
+    case 7: return launch_k<7>(p, in_dtype, x, out, rin, packed, stream);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t launch_planar_lowpass(const PlanarLowpass& p0, int in_dtype, const void* x, float* scratch, cudaStream_t stream) {
+  PlanarLowpass p = p0;
+  p.total = (long long)p.B * p.C * cdiv(p.H, 8) * cdiv(p.W, 8);
+  const long long want = (p.total + 255) / 256;
+  const unsigned blocks = (unsigned)(want > 148 * 64 ? 148 * 64 : want);
+  switch (in_dtype) {
+    case 0: wt2d_planar_lowpass_kernel<float><<<blocks, 256, 0, stream>>>(p, static_cast<const float*>(x), scratch); break;
+    case 1: wt2d_planar_lowpass_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(p, static_cast<const __nv_bfloat16*>(x), scratch); break;
+    default: wt2d_planar_lowpass_kernel<__half><<<blocks, 256, 0, stream>>>(p, static_cast<const __half*>(x), scratch); break;
+  }
+  return cudaGetLastError();
+}
+
+}  // namespace wt

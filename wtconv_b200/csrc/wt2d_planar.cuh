@@ -1,0 +1,719 @@
+// Planar kernels of the 2-D WTConv forward for sm_100a: whole planes with every level on chip, or halo tiles
+// of one level, for tensors of any layout (kernel sizes 3, 5, 7, any output stride).
+//
+// Replaces, for the planes of a CTA, wtconv/wtconv2d.py:46-85.  The tile kernels of wt2d_fused.cuh that did
+// this before spent 290 thread instructions per element on a path of 58 multiply-adds (28 x 28 planes, K = 5:
+// 125 us for 6.4 M elements, FMA pipe 21 % busy); what was changed and why:
+//
+//   * everything is planar fp32 in shared memory with zero borders that are cleared once: CTAs are
+//     persistent and later planes rewrite the interior only;
+//   * the pixels become the first level's sub-bands while they are loaded (one 2 x 2 block per step), so
+//     the frame is not read back for the first analysis;
+//   * a lane owns one sub-band of a tile of 4 x 4 positions: 16 accumulators and a K x K tap set in registers
+//     (kept over all its tiles), eight 16-byte window words per 100 multiply-adds at K = 5.  The four
+//     sub-bands of a tile sit in neighbouring lanes; two exchange steps with the synthesis butterfly
+//     (wavelet.py:70-75) folded in give each lane a 4 x 4 pixel quadrant of the tile, on which it then runs
+//     the base convolution with the same code.  One 400-FMA body serves every level and the base
+//     path, which keeps the kernel inside the instruction cache (the fully unrolled
+//     tile kernels lost a third of their cycles to instruction fetches);
+//   * reconstructions of deeper levels enter all four outputs of a position with a plus sign, so the levels
+//     do not wait for each other: level 2 and the chain of smaller ones (a warp per channel, no CTA
+//     barrier) run side by side and the top level adds both.
+#pragma once
+
+#include "wt2d_planar_host.h"
+
+namespace wt {
+
+#ifdef __CUDA_ARCH__
+// n / d for 0 <= n < 2^20 with inv = 1.f / d: exact, because (n + 1/2) / d is at least 1 / (2d) away from an
+// integer; a tenth of the instructions of an integer division (the phases of a small plane are short
+// enough for their set-up to matter)
+__device__ __forceinline__ int planar_div(int n, float inv) { return __float2int_rz(((float)n + 0.5f) * inv); }
+
+// 4 x 4 outputs of a K x K cross-correlation; p: top-left element of the window (16-byte aligned)
+template <int K>
+__device__ __forceinline__ void planar_conv(const float* __restrict__ p, int pitch, const float (&w)[K * K], float (&acc)[4][4]) {
+  constexpr int NV = (4 + K - 1 + 3) / 4;
+#pragma unroll
+  for (int iy = 0; iy < 4 + K - 1; ++iy) {
+    float row[4 * NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const float4 t = *reinterpret_cast<const float4*>(p + iy * pitch + 4 * v);
+      row[4 * v] = t.x; row[4 * v + 1] = t.y; row[4 * v + 2] = t.z; row[4 * v + 3] = t.w;
+    }
+#pragma unroll
+    for (int dy = 0; dy < K; ++dy) {
+      const int oy = iy - dy;
+      if (oy < 0 || oy >= 4) continue;
+#pragma unroll
+      for (int dx = 0; dx < K; ++dx)
+#pragma unroll
+        for (int ox = 0; ox < 4; ++ox) acc[oy][ox] = fmaf(w[dy * K + dx], row[ox + dx], acc[oy][ox]);
+    }
+  }
+}
+
+template <int K>
+__device__ __forceinline__ void planar_taps(const float* __restrict__ p, float (&w)[K * K]) {
+#pragma unroll
+  for (int v = 0; v < (K * K + 3) / 4; ++v) {
+    const float4 t = reinterpret_cast<const float4*>(p)[v];
+    const float q[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (4 * v + i < K * K) w[4 * v + i] = q[i];
+  }
+}
+
+// Synthesis over the four lanes of a tile.  In: lane s (low two bits) holds sub-band s at 4 x 4 positions.
+// Out: lane t = 2 ty + tx holds the 4 x 4 pixels of positions (2 ty .. +1, 2 tx .. +1):
+// pixel (2i + a, 2j + b) = LL + (-1)^a LH + (-1)^b HL + (-1)^(a+b) HH.  Step one exchanges column halves between
+// the sub-bands that differ in the row sign, step two row halves between those that differ in the column sign.
+__device__ __forceinline__ void planar_synthesis(const float (&v)[4][4], float (&o)[4][4], int lane) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const bool b0 = lane & 1, b1 = lane & 2;
+  const float s0 = b0 ? -1.f : 1.f, s1 = b1 ? -1.f : 1.f;
+  float m[2][4][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const float keep = b0 ? v[i][2 + q] : v[i][q];
+      const float r = __shfl_xor_sync(kFull, b0 ? v[i][q] : v[i][2 + q], 1);
+      m[0][i][q] = keep + r;
+      m[1][i][q] = (keep - r) * s0;
+    }
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const float keep = b1 ? m[a][2 + i][q] : m[a][i][q];
+        const float r = __shfl_xor_sync(kFull, b1 ? m[a][i][q] : m[a][2 + i][q], 2);
+        o[2 * i + a][2 * q] = keep + r;
+        o[2 * i + a][2 * q + 1] = (keep - r) * s1;
+      }
+}
+
+// Four pixels of a row starting at x (a multiple of VEC, as is W; zeros outside [0, W)) as raw words.
+// VEC: pixels per access; VEC = 1 takes any stride.
+template <typename T, int VEC>
+struct PlanarQuad {
+  typedef typename RawChunk<(VEC * (int)sizeof(T) < 4 ? 4 : VEC * (int)sizeof(T))>::type raw_t;
+  raw_t raw[4 / VEC];
+  __device__ __forceinline__ void load(const T* __restrict__ p, int x, int W, long long step, bool ok) {
+#pragma unroll
+    for (int k = 0; k < 4 / VEC; ++k) {
+      raw[k] = raw_t();                                         // zero bits are 0.0 in every type
+      const int xx = x + k * VEC;
+      if (!ok || xx < 0 || xx >= W) continue;
+      if (VEC > 1) raw[k] = __ldg(reinterpret_cast<const raw_t*>(p + xx));
+      else {
+        Chunk<T, 4> c;
+        c.raw = 0u;
+        c.set(0, p[(long long)xx * step]);
+        *reinterpret_cast<unsigned*>(&raw[k]) = c.raw;
+      }
+    }
+  }
+  __device__ __forceinline__ float get(int i) const {
+    Chunk<T, (VEC * (int)sizeof(T) < 4 ? 4 : VEC * (int)sizeof(T))> c;
+    c.raw = raw[i / VEC];
+    return Elem<T>::to_f(c.get(i % VEC));
+  }
+};
+
+__device__ __forceinline__ void planar_haar(float a, float b, float c, float d, float (&s)[4]) {
+  const float pp = a + b, qq = a - b, uu = c + d, vv = c - d;
+  s[0] = pp + uu; s[1] = pp - uu; s[2] = qq + vv; s[3] = qq - vv;
+}
+
+// Lanes over the columns of flattened (channel, row) pairs: 2^shift >= min(ncols, 32) lanes per row
+struct PlanarWalk {
+  int shift, col, row, step;
+  __device__ __forceinline__ PlanarWalk(int ncols, int tid, int nthr) {
+    shift = ncols > 16 ? 5 : 32 - __clz(imax(ncols, 1) - 1);
+    col = tid & ((1 << shift) - 1);
+    row = tid >> shift;
+    step = nthr >> shift;
+  }
+};
+
+// Fill of a CTA's planes: pixels -> pixel frame (with the base path) and sub-bands of the first level.
+// (ra, rb) x (ca, cb): rows and columns of the sub-band frame to write; frame cell (r, c) is position
+// (py0 + r, px0 + c) of level 1, its pixels rows 2r - HS, 2r - HS + 1 of the pixel frame.
+// SHIFT = 1: the plane of the stage is the low-pass plane one level below the tensor read; its values are
+// formed as 2 x 2 sums while loading (wtconv2d.py:49-54), which reads no more bytes than a stored fp32 plane
+// would take and saves writing it.
+template <typename T, int K, bool FINAL, int SHIFT>
+struct PlanarFill {
+  const PlanarStage& p;
+  float* sm;
+  const T* src;                       // first channel of the group, sample n
+  int gc;                             // channels present
+  int py0, px0, ra, rb, ca, cb;
+  float inv_nr;                       // 1 / (rb - ra)
+  static constexpr int HS = K / 2;
+
+  __device__ __forceinline__ void put_pixels(int g, int r, int dy, int c, float v0, float v1) const {
+    const int fr = 2 * r - HS + dy, fc = 2 * c - HS;
+    float* d = sm + p.xoff + g * p.xplane + fr * p.xpitch + fc;
+    if (!p.tiled) {                    // interior positions only: always inside the frame
+      if (HS % 2 == 0) *reinterpret_cast<float2*>(d) = make_float2(v0, v1);
+      else { d[0] = v0; d[1] = v1; }
+      return;
+    }
+    if (fr < 0 || fr >= p.xrows) return;
+    if (HS % 2 == 0) {
+      if (fc >= 0 && fc < p.xcols) *reinterpret_cast<float2*>(d) = make_float2(v0, v1);
+    } else {
+      if (fc >= 0 && fc < p.xcols) d[0] = v0;
+      if (fc + 1 >= 0 && fc + 1 < p.xcols) d[1] = v1;
+    }
+  }
+
+  // two neighbouring cells of a frame row
+  static __device__ __forceinline__ void put2(float* d, float v0, float v1) {
+    if (HS % 2 == 0) *reinterpret_cast<float2*>(d) = make_float2(v0, v1);
+    else { d[0] = v0; d[1] = v1; }
+  }
+
+  // Rows of any layout: one item = two positions (2 x 4 pixels) of one channel.  Lanes run over the columns of
+  // a row; a thread keeps its column and walks down the flattened (channel, row) pairs with three running
+  // offsets (source, pixel frame, sub-bands), the next row's pixels on their way while it works on a row.
+  template <int VEC>
+  __device__ __forceinline__ void rows(int tid, int nthr) const {
+    const int H = p.Hsrc, W = p.Wsrc;
+    const int ncols = (cb - ca + 1) / 2, nr = rb - ra;
+    const PlanarWalk wk(ncols, tid, nthr);
+    const int nrows = gc * nr;
+    const int g0 = planar_div(wk.row, inv_nr), r0 = wk.row - g0 * nr;
+    const int dg = planar_div(wk.step, inv_nr), dr = wk.step - dg * nr;
+    const int s1 = (int)p.xs[1], s2 = (2 << SHIFT) * (int)p.xs[2];              // source steps of a channel and of a position row
+    const int splane = p.splane[1], spitch = p.spitch[1];
+    for (int ci = wk.col; ci < ncols; ci += 32) {
+      const int c = ca + 2 * ci, x = (2 << SHIFT) * (px0 + c);
+      const bool two = c + 1 < cb;
+      int r = r0, y = (2 << SHIFT) * (py0 + ra + r0);
+      int so = g0 * s1 + r0 * s2 + (2 << SHIFT) * (py0 + ra) * (int)p.xs[2];
+      int sf = p.soff[1] + 4 * g0 * splane + (ra + r0) * spitch + c;
+      int xf = p.xoff + g0 * p.xplane + (2 * (ra + r0) - HS) * p.xpitch + 2 * c - HS;
+      constexpr int NR = 2 << SHIFT;
+      PlanarQuad<T, VEC> q[NR][1 << SHIFT];
+      auto fetch = [&](bool more) {
+#pragma unroll
+        for (int k = 0; k < NR; ++k)
+#pragma unroll
+          for (int h = 0; h < (1 << SHIFT); ++h)
+            q[k][h].load(src + so + k * (int)p.xs[2], x + 4 * h, W, p.xs[3], more && y + k >= 0 && y + k < H);
+      };
+      fetch(wk.row < nrows);
+      for (int row = wk.row; row < nrows; row += wk.step) {
+        float v[2][4];
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (SHIFT == 0) v[k][i] = q[k][0].get(i);
+            else {
+              const int h = (2 * i / 4) & ((1 << SHIFT) - 1), e = 2 * i % 4;
+              v[k][i] = (q[(2 * k) % NR][h].get(e) + q[(2 * k) % NR][h].get((e + 1) % 4)) +
+                        (q[(2 * k + 1) % NR][h].get(e) + q[(2 * k + 1) % NR][h].get((e + 1) % 4));
+            }
+          }
+        const int sf0 = sf, xf0 = xf, fr = 2 * (ra + r) - HS;
+        // next row
+        r += dr; y += dr * NR;
+        so += dg * s1 + dr * s2; sf += dg * 4 * splane + dr * spitch; xf += dg * p.xplane + 2 * dr * p.xpitch;
+        if (r >= nr) {
+          r -= nr; y -= nr * NR;
+          so += s1 - nr * s2; sf += 4 * splane - nr * spitch; xf += p.xplane - 2 * nr * p.xpitch;
+        }
+        fetch(row + wk.step < nrows);
+        if (FINAL) {
+          if (!p.tiled) {                                       // interior positions only: always inside the frame
+            put2(sm + xf0, v[0][0], v[0][1]);
+            put2(sm + xf0 + p.xpitch, v[1][0], v[1][1]);
+            if (two) {
+              put2(sm + xf0 + 2, v[0][2], v[0][3]);
+              put2(sm + xf0 + p.xpitch + 2, v[1][2], v[1][3]);
+            }
+          } else {
+            const int fc = 2 * c - HS;
+#pragma unroll
+            for (int k = 0; k < 2; ++k)
+              if (fr + k >= 0 && fr + k < p.xrows) {
+#pragma unroll
+                for (int i = 0; i < 4; i += 2) {
+                  float* d = sm + xf0 + k * p.xpitch + i;
+                  if (fc + i >= 0 && fc + i + 1 < p.xcols) put2(d, v[k][i], v[k][i + 1]);
+                  else if (HS % 2) {
+                    if (fc + i >= 0 && fc + i < p.xcols) d[0] = v[k][i];
+                    if (fc + i + 1 >= 0 && fc + i + 1 < p.xcols) d[1] = v[k][i + 1];
+                  }
+                }
+              }
+          }
+        }
+        if (p.nlev > 0) {
+          float a[4], b[4];
+          planar_haar(v[0][0], v[0][1], v[1][0], v[1][1], a);
+          planar_haar(v[0][2], v[0][3], v[1][2], v[1][3], b);
+          float* d = sm + sf0;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if (two) put2(d, a[k], b[k]);
+            else d[0] = a[k];
+            d += splane;
+          }
+        }
+      }
+    }
+  }
+
+  // channel chunks: one item = V channels of one position
+  template <int CB>
+  __device__ __forceinline__ void chunks(int tid, int nthr) const {
+    constexpr int V = CB / (int)sizeof(T);
+    const int H = p.Hsrc, W = p.Wsrc;
+    const int nch = p.G / V, ncols = cb - ca;
+    const PlanarWalk wk(ncols, tid, nthr);
+    const int nr = rb - ra, nrows = nch * nr;
+    for (int row = wk.row; row < nrows; row += wk.step) {
+      const int ch = planar_div(row, inv_nr), r = ra + row - ch * nr;          // chunk slowest: a warp covers neighbouring pixels
+      const int y = (2 << SHIFT) * (py0 + r);
+      for (int c = ca + wk.col; c < cb; c += 32) {
+        const int x = (2 << SHIFT) * (px0 + c);
+        float v[2][2][V];
+#pragma unroll
+        for (int by = 0; by < 2; ++by)
+#pragma unroll
+          for (int bx = 0; bx < 2; ++bx) {
+            if (SHIFT == 0) {
+              Chunk<T, CB> q = load<CB>(y + by, x + bx, H, W, ch);
+#pragma unroll
+              for (int e = 0; e < V; ++e) v[by][bx][e] = Elem<T>::to_f(q.get(e));
+            } else {
+              const int yy = y + 2 * by, xx = x + 2 * bx;
+              const Chunk<T, CB> q0 = load<CB>(yy, xx, H, W, ch), q1 = load<CB>(yy, xx + 1, H, W, ch);
+              const Chunk<T, CB> q2 = load<CB>(yy + 1, xx, H, W, ch), q3 = load<CB>(yy + 1, xx + 1, H, W, ch);
+#pragma unroll
+              for (int e = 0; e < V; ++e)
+                v[by][bx][e] = (Elem<T>::to_f(q0.get(e)) + Elem<T>::to_f(q1.get(e))) + (Elem<T>::to_f(q2.get(e)) + Elem<T>::to_f(q3.get(e)));
+            }
+          }
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          const int g = ch * V + e;
+          const float a = v[0][0][e], b = v[0][1][e], cc = v[1][0][e], d = v[1][1][e];
+          if (FINAL) { put_pixels(g, r, 0, c, a, b); put_pixels(g, r, 1, c, cc, d); }
+          if (p.nlev > 0) {
+            float s[4];
+            planar_haar(a, b, cc, d, s);
+            float* o = sm + p.soff[1] + (4 * g) * p.splane[1] + r * p.spitch[1] + c;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) o[k * p.splane[1]] = s[k];
+          }
+        }
+      }
+    }
+  }
+
+  template <int CB>
+  __device__ __forceinline__ Chunk<T, CB> load(int y, int x, int H, int W, int ch) const {
+    typedef typename RawChunk<CB>::type raw_t;
+    Chunk<T, CB> q;
+    q.raw = raw_t();                                            // zero bits are 0.0 in every type
+    if (y >= 0 && y < H && x >= 0 && x < W)
+      q.raw = __ldg(reinterpret_cast<const raw_t*>(src + (long long)y * p.xs[2] + (long long)x * p.xs[3] + ch * (CB / (int)sizeof(T))));
+    return q;
+  }
+
+  __device__ __forceinline__ void run(int tid, int nthr) const {
+    if (p.xchunk * (int)sizeof(T) == 16 && gc == p.G) chunks<16>(tid, nthr);
+    else if (p.xchunk * (int)sizeof(T) == 8 && gc == p.G) chunks<8>(tid, nthr);
+    else if (p.xchunk * (int)sizeof(T) == 4 && gc == p.G) chunks<4>(tid, nthr);
+    else if (p.xvec >= 4 && p.Wsrc % 4 == 0 && (HS % 2 == 0 || SHIFT || !p.tiled)) rows<4>(tid, nthr);   // (odd halo: a tile starts two pixels off)
+    else if (p.xvec >= 2 && p.Wsrc % 2 == 0) rows<2>(tid, nthr);
+    else rows<1>(tid, nthr);
+  }
+};
+
+// Analysis of level j >= 2 for channels g0 .. g0+ng-1: low-pass band of level j-1 -> sub-bands of level j
+template <int K>
+__device__ __forceinline__ void planar_analysis(const PlanarStage& p, float* sm, int j, int g0, int ng, int tid, int nthr) {
+  constexpr int HS = K / 2;
+  const int hj = p.h[j], wj = p.w[j], sp = p.spitch[j - 1], dp = p.spitch[j], plane = p.splane[j];
+  const PlanarWalk wk(wj, tid, nthr);
+  const int nrows = ng * hj;
+  const float inv = p.inv_h[j];
+  int g = planar_div(wk.row, inv), r = wk.row - g * hj;
+  const int dg = planar_div(wk.step, inv), dr = wk.step - dg * hj;
+  for (int row = wk.row; row < nrows; row += wk.step) {
+    const float* src = sm + p.soff[j - 1] + 4 * (g0 + g) * p.splane[j - 1] + (2 * r + HS) * sp + HS;
+    float* dst = sm + p.soff[j] + 4 * (g0 + g) * plane + (r + HS) * dp + HS;
+    for (int c = wk.col; c < wj; c += 32) {
+      float a, b, cc, d, s[4];
+      if (HS % 2 == 0) {
+        const float2 t0 = *reinterpret_cast<const float2*>(src + 2 * c), t1 = *reinterpret_cast<const float2*>(src + sp + 2 * c);
+        a = t0.x; b = t0.y; cc = t1.x; d = t1.y;
+      } else {
+        a = src[2 * c]; b = src[2 * c + 1]; cc = src[sp + 2 * c]; d = src[sp + 2 * c + 1];
+      }
+      planar_haar(a, b, cc, d, s);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) dst[k * plane + c] = s[k];
+    }
+    g += dg; r += dr;
+    if (r >= hj) { r -= hj; ++g; }
+  }
+}
+
+// One 4 x 4 tile of a level below the top (built once per CTA, in shared memory)
+__device__ __forceinline__ unsigned planar_smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+constexpr unsigned kPlanarWaitSpins = 1u << 14;   // bound of the wait for the other warps' deep tiles
+
+struct PlanarTile {
+  int win, pitch, plane, taps;          // window of sub-band 0 of channel 0, its pitch and plane size, tap set of sub-band 0
+  int out, opitch, oplane, pad;         // 8 x 8 block of the reconstruction of channel 0, its pitch and plane size
+};
+#endif
+
+// Registers: 16 accumulators, 16 exchanged values, K*K taps, one window row and the addresses; three CTAs
+// of eight warps share an SM at K = 3 and 5 (80 registers), two at K = 7.
+template <typename T, typename TO, int K, bool FINAL>
+__global__ void __launch_bounds__(kPlanarMaxThreads, planar_ctas(K))
+wt2d_planar_kernel(const __grid_constant__ PlanarStage p, const T* __restrict__ x, TO* __restrict__ y,
+                   const float* __restrict__ rin, const float* __restrict__ packed) {
+#ifdef __CUDA_ARCH__
+  extern __shared__ __align__(128) float planar_smem[];
+  float* const sm = planar_smem;
+  constexpr int HS = K / 2;
+  const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarp = nthr >> 5;
+  const int s = lane & 3, u = lane >> 2;
+  const int ts = tapset_floats(K, 2);
+  PlanarTile* const tiles = reinterpret_cast<PlanarTile*>(sm + p.tileoff);
+  float* const deep_done = sm + p.tileoff + 8 * p.ntiles;   // mbarrier: completes when every warp has left the deep tiles of an item
+  if (tid == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(planar_smem_addr(deep_done)), "r"(nwarp) : "memory");
+  for (int i = tid; i < p.zero_floats / 4; i += nthr) reinterpret_cast<float4*>(sm)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  {
+    int first = 0;
+    for (int j = 2; j <= p.nlev; ++j) {
+      const int nt = p.tyn[j] * p.txn[j];
+      for (int t = tid; t < nt; t += nthr) {
+        const int ty = t / p.txn[j], tx = t - ty * p.txn[j];
+        PlanarTile d;
+        d.win = p.soff[j] + 4 * ty * p.spitch[j] + 4 * tx; d.pitch = p.spitch[j]; d.plane = p.splane[j];
+        d.taps = ts * (p.has_base + 4 * (j - 1));
+        d.out = p.eoff[j - 1] + 8 * ty * p.epitch[j - 1] + 8 * tx; d.opitch = p.epitch[j - 1]; d.oplane = p.eplane[j - 1];
+        d.pad = 0;
+        tiles[first + t] = d;
+      }
+      first += nt;
+    }
+  }
+  __syncthreads();
+  int loaded = -1;
+  unsigned parity = 0;
+  for (unsigned item = blockIdx.x; item < (unsigned)p.total; item += gridDim.x) {
+    const unsigned rest = item / (unsigned)p.ngroups;
+    const int cg = (int)(item - rest * (unsigned)p.ngroups);
+    int tile_y = 0, tile_x = 0, n = (int)rest;
+    if (p.tiled) {
+      const unsigned t = rest / (unsigned)p.ntx;
+      tile_x = (int)(rest - t * (unsigned)p.ntx);
+      n = (int)(t / (unsigned)p.nty);
+      tile_y = (int)(t - (unsigned)n * (unsigned)p.nty);
+    }
+    const int c0 = cg << p.gshift, gc = imin(p.G, p.C - c0);
+    const int Y0 = tile_y * p.TH, X0 = tile_x * p.TW;
+    if (cg != loaded) {
+      const int per = p.wlen / 4;
+      for (int i = tid; i < gc * per; i += nthr) {
+        const int g = i / per, k = i - g * per;
+        async_copy16(sm + p.woff + g * p.wchan + 4 * k, packed + (size_t)(c0 + g) * p.wstride + p.wbeg + 4 * k);
+      }
+      loaded = cg;
+    }
+    {
+      PlanarFill<T, K, FINAL, 0> f{p, sm, x + (long long)n * p.xs[0] + (long long)c0 * p.xs[1], gc, Y0 - HS, X0 - HS, 0, 0, 0, 0, 0.f};
+      if (p.tiled) {           // the whole frame, halo included
+        f.rb = 4 * p.tyn[1] + 2 * HS; f.cb = 4 * p.txn[1] + 2 * HS;
+      } else {                 // the borders stay zero
+        f.ra = HS; f.rb = HS + (p.h[0] + 1) / 2; f.ca = HS; f.cb = HS + (p.w[0] + 1) / 2;
+      }
+      f.inv_nr = p.inv_rows;
+      if (FINAL || p.shift == 0) {
+        f.run(tid, nthr);
+      } else if constexpr (!FINAL) {
+        PlanarFill<T, K, false, 1> f1{p, sm, f.src, gc, f.py0, f.px0, f.ra, f.rb, f.ca, f.cb, f.inv_nr};
+        f1.run(tid, nthr);
+      }
+    }
+    async_wait_all();
+    __syncthreads();
+    // ---- analyses below the first level: CTA-wide while the planes are large, then a warp per channel
+    if (p.nlev > 1) {
+      for (int j = 2; j < p.jlocal; ++j) {
+        planar_analysis<K>(p, sm, j, 0, gc, tid, nthr);
+        __syncthreads();
+      }
+      if (p.jlocal <= p.nlev) {
+        for (int g = warp; g < gc; g += nwarp)
+          for (int j = p.jlocal; j <= p.nlev; ++j) {
+            planar_analysis<K>(p, sm, j, g, 1, lane, 32);
+            __syncwarp();
+          }
+        __syncthreads();
+      }
+    }
+
+    // ---- convolutions and synthesis: phase 0 every tile of the levels below the top, phase 1 the top level
+    // and the base path.  The levels are independent of one another (see the top of the file).
+    const int gp = imin(p.G, 8), gpl = imin(p.gshift, 3), ngl = p.gshift - gpl, tpw = 8 >> gpl;
+    bool waiting = p.nlev > 1;
+#pragma unroll 1
+    for (int phase = p.nlev > 1 ? 0 : 1; phase < 2; ++phase) {
+      const int ntile = phase ? p.tyn[1] * p.txn[1] : p.ntiles;
+      const int slots = ((ntile + tpw - 1) >> (3 - gpl)) << ngl;
+#pragma unroll 1
+      for (int slot = warp; slot < slots; slot += nwarp) {
+        const int tq = ((slot >> ngl) << (3 - gpl)) + (u >> gpl), t = imin(tq, ntile - 1);
+        const int g = (slot & ((1 << ngl) - 1)) * 8 + (u & (gp - 1));
+        const bool live = tq < ntile && g < gc;
+        const float* win;
+        const float* tap = sm + p.woff + g * p.wchan;
+        float* out = nullptr;
+        int pitch, opitch = 0, ty = 0, tx = 0;
+        if (phase) {
+          ty = planar_div(t, p.inv_txn); tx = t - ty * p.txn[1];
+          win = sm + p.soff[1] + (4 * g + s) * p.splane[1] + 4 * ty * p.spitch[1] + 4 * tx;
+          pitch = p.spitch[1];
+          tap += ts * (p.has_base + s);
+        } else {
+          const int4 d0 = *reinterpret_cast<const int4*>(&tiles[t]), d1 = *(reinterpret_cast<const int4*>(&tiles[t]) + 1);
+          win = sm + d0.x + (4 * g + s) * d0.z;
+          pitch = d0.y;
+          tap += d0.w + ts * s;
+          opitch = d1.y;
+          out = sm + d1.x + g * d1.z + 4 * (s >> 1) * opitch + 4 * (s & 1);
+        }
+        float acc[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) acc[i][q] = 0.f;
+        const int fy = 8 * ty + 4 * (s >> 1), fx = 8 * tx + 4 * (s & 1);
+        // pass 0: the sub-band; pass 1: the base path on the quadrant the synthesis leaves in this lane (the
+        // only pass of a layer without levels)
+        if (p.nlev == 0) {
+          tap = sm + p.woff + g * p.wchan;
+          win = sm + p.xoff + g * p.xplane + fy * p.xpitch + fx;
+          pitch = p.xpitch;
+          const float bias = tap[K * K];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[i][q] = bias;
+        }
+#pragma unroll 1
+        for (int pass = p.nlev == 0 ? 1 : 0;; ++pass) {
+          float w[K * K];
+          planar_taps<K>(tap, w);
+          planar_conv<K>(win, pitch, w, acc);
+          if (pass == 0) planar_synthesis(acc, acc, lane);
+          if (phase == 0 || !FINAL || pass == 1) break;
+          tap = sm + p.woff + g * p.wchan;
+          win = sm + p.xoff + g * p.xplane + fy * p.xpitch + fx;
+          pitch = p.xpitch;
+        }
+        if (phase && p.nlev > 0) {
+          if (waiting) {               // the other warps' deep tiles (they were started before this warp's top level)
+            for (unsigned spin = 0; spin < kPlanarWaitSpins; ++spin) {
+              unsigned done;
+              asm volatile("{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                           : "=r"(done) : "r"(planar_smem_addr(deep_done)), "r"(parity) : "memory");
+              if (done) break;
+            }
+            waiting = false;
+          }
+          // What is the same for the 2 x 2 pixels of a position: the reconstructions of the deeper levels
+          // (wtconv2d.py:71; plane m is 2^(m-1) times coarser) and the bias
+          float all = 0.f, add[2][2];
+          if (FINAL) all = sm[p.woff + g * p.wchan + K * K];
+          const int qy = 4 * ty + 2 * (s >> 1), qx = 4 * tx + 2 * (s & 1);
+          for (int m = 2; m < p.nlev; ++m) all += sm[p.eoff[m] + g * p.eplane[m] + (qy >> (m - 1)) * p.epitch[m] + (qx >> (m - 1))];
+          add[0][0] = add[0][1] = add[1][0] = add[1][1] = all;
+          if (p.nlev > 1) {
+            const float* e = sm + p.eoff[1] + g * p.eplane[1] + qy * p.epitch[1] + qx;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              const float2 v = *reinterpret_cast<const float2*>(e + i * p.epitch[1]);
+              add[i][0] += v.x; add[i][1] += v.y;
+            }
+          }
+          if (rin && live) {
+            const int hy = Y0 + qy, hx = X0 + qx;
+            const float* r = rin + (long long)n * p.rs[0] + (long long)(c0 + g) * p.rs[1] + (long long)hy * p.rs[2] + (long long)hx * p.rs[3];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              if (hy + i >= p.h[1]) break;
+              const float* ri = r + (long long)i * p.rs[2];
+              if (p.rvec && hx + 2 <= p.w[1]) {
+                const float2 v = __ldg(reinterpret_cast<const float2*>(ri));
+                add[i][0] += v.x; add[i][1] += v.y;
+              } else {
+                if (hx < p.w[1]) add[i][0] += __ldg(ri);
+                if (hx + 1 < p.w[1]) add[i][1] += __ldg(ri + p.rs[3]);
+              }
+            }
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[i][q] += add[i >> 1][q >> 1];
+        }
+        if (!live) continue;
+        if (phase == 0) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(out + i * opitch) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+          continue;
+        }
+        // ---- store (cropped to the plane: wtconv2d.py:76; strided: :84-85)
+        const int yy = 2 * Y0 + fy, xx = 2 * X0 + fx;
+        TO* ob = y + (long long)n * p.ys[0] + (long long)(c0 + g) * p.ys[1];
+        if (p.yvec >= 4 && p.out_stride == 1 && yy + 4 <= p.h[0] && xx + 4 <= p.w[0]) {
+          TO* o4 = ob + (yy * (int)p.ys[2] + xx);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            Chunk<TO, 4 * (int)sizeof(TO)> c;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) c.set(q, Elem<TO>::from_f(acc[i][q]));
+            *reinterpret_cast<typename RawChunk<4 * (int)sizeof(TO)>::type*>(o4) = c.raw;
+            o4 += (int)p.ys[2];
+          }
+        } else if (p.out_stride == 1 && yy + 4 <= p.h[0] && xx + 4 <= p.w[0]) {
+          // channels-last (the eight channels of a warp are neighbours) and rows that are not aligned
+          TO* o4 = ob + (yy * (int)p.ys[2] + xx * (int)p.ys[3]);
+          const int step = (int)p.ys[3];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            TO* o1 = o4;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) { *o1 = Elem<TO>::from_f(acc[i][q]); o1 += step; }
+            o4 += (int)p.ys[2];
+          }
+        } else if (p.out_stride == 1) {
+          ob += (long long)yy * p.ys[2] + (long long)xx * p.ys[3];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (yy + i >= p.h[0]) break;
+            TO* o4 = ob + (long long)i * p.ys[2];
+            if (p.yvec >= 2 && xx + 4 <= p.w[0]) {
+#pragma unroll
+              for (int q = 0; q < 4; q += 2) {
+                Chunk<TO, 2 * (int)sizeof(TO)> c;
+                c.set(0, Elem<TO>::from_f(acc[i][q])); c.set(1, Elem<TO>::from_f(acc[i][q + 1]));
+                *reinterpret_cast<typename RawChunk<2 * (int)sizeof(TO)>::type*>(o4 + q) = c.raw;
+              }
+            } else {
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                if (xx + q < p.w[0]) o4[(long long)q * p.ys[3]] = Elem<TO>::from_f(acc[i][q]);
+            }
+          }
+        } else {
+          const int st = p.out_stride;
+          int oy = (yy + st - 1) / st, ni = oy * st - yy;            // next stored row of the quadrant
+          const int ox0 = (xx + st - 1) / st, nq0 = ox0 * st - xx;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (i != ni) continue;
+            if (yy + i < p.h[0]) {
+              int nq = nq0;
+              TO* o1 = ob + (long long)oy * p.ys[2] + (long long)ox0 * p.ys[3];
+#pragma unroll
+              for (int q = 0; q < 4; ++q) {
+                if (q != nq) continue;
+                if (xx + q < p.w[0]) *o1 = Elem<TO>::from_f(acc[i][q]);
+                nq += st; o1 += p.ys[3];
+              }
+            }
+            ni += st; ++oy;
+          }
+        }
+      }
+      if (phase == 0) {
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(planar_smem_addr(deep_done)) : "memory");
+      }
+    }
+    if (p.nlev > 1) parity ^= 1u;
+    __syncthreads();           // the frames are rewritten by the next item
+  }
+#endif
+}
+
+// One thread = one 8 x 8 pixel block of one channel: sums over 2 x 2, 4 x 4 and 8 x 8 blocks
+template <typename T>
+__global__ void __launch_bounds__(256) wt2d_planar_lowpass_kernel(const __grid_constant__ PlanarLowpass a, const T* __restrict__ x, float* __restrict__ out) {
+#ifdef __CUDA_ARCH__
+  const unsigned bw = (unsigned)(a.W + 7) / 8, bh = (unsigned)(a.H + 7) / 8;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.total; i += (long long)gridDim.x * blockDim.x) {
+    unsigned bx, by, c, n;
+    if (a.cl) {
+      unsigned t = (unsigned)(i / a.C);
+      c = (unsigned)(i - (long long)t * a.C);
+      bx = t % bw; t /= bw;
+      by = t % bh; n = t / bh;
+    } else {
+      long long t = i / bw;
+      bx = (unsigned)(i - t * bw);
+      by = (unsigned)(t % bh);
+      t /= bh;
+      c = (unsigned)(t % a.C); n = (unsigned)(t / a.C);
+    }
+    const T* p = x + (long long)n * a.xs[0] + (long long)c * a.xs[1];
+    const int y0 = 8 * by, x0 = 8 * bx;
+    // output strides: (B, C, h, w) or (B, h, w, C)
+    auto put = [&](int k, int yy, int xx, float v) {
+      const int h = (a.H + (1 << k) - 1) >> k, w = (a.W + (1 << k) - 1) >> k;
+      if (a.off[k - 1] < 0 || yy >= h || xx >= w) return;
+      const long long at = a.cl ? (((long long)n * h + yy) * w + xx) * a.C + c : (((long long)n * a.C + c) * h + yy) * w + xx;
+      out[a.off[k - 1] + at] = v;
+    };
+    float s3 = 0.f, s2[2] = {0.f, 0.f};
+#pragma unroll
+    for (int ry = 0; ry < 4; ++ry) {
+      float v[2][8];
+#pragma unroll
+      for (int dy = 0; dy < 2; ++dy)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int yy = y0 + 2 * ry + dy, xx = x0 + q;
+          v[dy][q] = (yy < a.H && xx < a.W) ? Elem<T>::to_f(p[(long long)yy * a.xs[2] + (long long)xx * a.xs[3]]) : 0.f;
+        }
+      float s1[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        s1[q] = (v[0][2 * q] + v[0][2 * q + 1]) + (v[1][2 * q] + v[1][2 * q + 1]);
+        put(1, 4 * by + ry, 4 * bx + q, s1[q]);
+      }
+      s2[0] += s1[0] + s1[1];
+      s2[1] += s1[2] + s1[3];
+      if (ry & 1) {
+        put(2, 2 * by + ry / 2, 2 * bx, s2[0]);
+        put(2, 2 * by + ry / 2, 2 * bx + 1, s2[1]);
+        s3 += s2[0] + s2[1];
+        s2[0] = s2[1] = 0.f;
+      }
+    }
+    put(3, by, bx, s3);
+  }
+#endif
+}
+
+}  // namespace wt

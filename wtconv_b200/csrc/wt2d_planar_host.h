@@ -1,0 +1,150 @@
+// Launch description and planner of the planar kernels (see wt2d_planar.cuh): plain data and host-side
+// geometry, usable without any CUDA device code.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "wt_common.h"
+
+namespace wt {
+
+constexpr int kPlanarMaxLev = 8;       // levels a whole-plane stage can hold on chip
+constexpr int kPlanarMaxThreads = 256;
+WT_HD constexpr int planar_ctas(int K) { return K <= 5 ? 3 : 2; }   // CTAs of 256 threads per SM the registers allow
+
+// One stage: `nlev` levels on whole planes, or one level (or the base path alone) on halo tiles.
+// Level j = 1..nlev of the stage is layer level lvl0 + j; plane j is h[j] x w[j] (plane 0 is the one read).
+// All offsets, pitches and plane sizes are in floats.
+struct PlanarStage {
+  int B, C;
+  int K, nlev, lvl0, has_base, tiled;
+  int G, gshift, ngroups;                 // channels per CTA (a power of two)
+  int TH, TW, nty, ntx;                   // level-1 positions per CTA, CTAs per plane
+  int h[kPlanarMaxLev + 1], w[kPlanarMaxLev + 1];
+  int tyn[kPlanarMaxLev + 1], txn[kPlanarMaxLev + 1];      // thread tiles (4 x 4 positions) of a level
+  int xoff, xpitch, xplane, xrows, xcols;                  // pixel frame (only with the base path)
+  int soff[kPlanarMaxLev + 1], spitch[kPlanarMaxLev + 1], splane[kPlanarMaxLev + 1];   // sub-band s of channel g: soff + (4 g + s) splane
+  int eoff[kPlanarMaxLev + 1], epitch[kPlanarMaxLev + 1], eplane[kPlanarMaxLev + 1];   // reconstruction of plane j by level j + 1
+  int woff, wchan, wlen, wbeg, wstride;   // staged tap sets: per channel wlen floats from wbeg of the packed block
+  int zero_floats;                        // frames to clear once
+  float inv_rows, inv_txn, inv_h[kPlanarMaxLev + 1];       // reciprocals of the fill's rows, txn[1] and h[j]
+  int jlocal;                             // from this level on the analyses run warp by warp (at most 64 positions per plane)
+  int tileoff, ntiles;                    // descriptors of the tiles below the top level
+  int shift, Hsrc, Wsrc;                  // 1: plane 0 is the 2 x 2 block sums of the Hsrc x Wsrc tensor read (else plane 0 itself)
+  int nthreads, smem_bytes, grid;
+  double score;                           // planner's estimate of the busy warps per SM
+  long long total;                        // work items: samples x tiles x channel groups
+  long long xs[4], ys[4], rs[4];          // element strides (n, c, row, col): input, output, deeper reconstruction
+  int out_stride, Ho, Wo;
+  int xvec, xchunk, yvec, rvec;           // pixels of a row per access (rvec: two may be read at once); channels per access (0: none)
+};
+
+inline int planar_resident(const PlanarStage& p) {          // CTAs per SM
+  const int by_smem = (228 * 1024) / (p.smem_bytes + 1024), by_regs = planar_ctas(p.K) * kPlanarMaxThreads / p.nthreads;
+  return imax(1, imin(by_smem, by_regs));
+}
+
+// Fills the geometry of a stage; returns its dynamic shared memory in bytes.
+// Plane sizes, K, nlev, lvl0, has_base, tiled, G, TH, TW must be set.
+inline long long planar_layout(PlanarStage& p) {
+  const int HS = p.K / 2, NV = (4 + p.K - 1 + 3) / 4;      // halo, 16-byte words of a window row
+  const int d = p.nlev;
+  p.ngroups = cdiv(p.C, p.G);
+  p.gshift = 0;
+  while ((1 << p.gshift) < p.G) ++p.gshift;
+  const int h1 = cdiv(p.h[0], 2), w1 = cdiv(p.w[0], 2);
+  p.nty = cdiv(h1, p.TH);
+  p.ntx = cdiv(w1, p.TW);
+  auto pad = [](long long n, int want) {                   // smallest n' >= n with n' % 32 == want (all multiples of 4)
+    n = (n + 3) / 4 * 4;
+    while (n % 32 != want) n += 4;
+    return n;
+  };
+  long long off = 0;
+  // Quarter warps hold four sub-bands (or four quadrants) x two channels, or x two neighbouring tiles with one
+  // channel per CTA.  Plane sizes of 4 mod 32 floats (8 with one channel) put those eight windows into
+  // different 16-byte bank groups; for the pixel frame and the reconstructions (quadrants: 4 columns, 4 rows)
+  // pitches of 4 mod 8 and planes of 8 mod 32 do.
+  for (int j = 1; j <= imax(d, 1); ++j) {
+    const int hh = j == 1 ? imin(p.TH, h1) : p.h[j], ww = j == 1 ? imin(p.TW, w1) : p.w[j];
+    p.tyn[j] = cdiv(hh, 4);
+    p.txn[j] = cdiv(ww, 4);
+    p.spitch[j] = 4 * (p.txn[j] - 1) + 4 * NV;
+    p.splane[j] = (int)pad((long long)(4 * p.tyn[j] + 2 * HS) * p.spitch[j], p.G == 1 ? 8 : 4);
+    p.soff[j] = (int)off;
+    if (j <= d) off += (long long)p.G * 4 * p.splane[j];
+  }
+  p.xrows = 8 * p.tyn[1] + 2 * HS;
+  p.xcols = 8 * p.txn[1] - 4 + 4 * NV;
+  p.xpitch = p.xcols + ((p.xcols / 4) % 2 == 0 ? 4 : 0);
+  p.xplane = (int)pad((long long)p.xrows * p.xpitch, 8);
+  p.xoff = (int)off;
+  if (p.has_base) off += (long long)p.G * p.xplane;
+  p.jlocal = d + 1;
+  for (int j = d; j >= 2 && p.h[j] * p.w[j] <= 64; --j) p.jlocal = j;
+  for (int j = 1; j < d; ++j) {
+    const int cols = 8 * p.txn[j + 1];
+    p.epitch[j] = cols + 4;
+    p.eplane[j] = (int)pad((long long)8 * p.tyn[j + 1] * p.epitch[j], 8);
+    p.eoff[j] = (int)off;
+    off += (long long)p.G * p.eplane[j];
+  }
+  p.zero_floats = (int)((off + 3) / 4 * 4);
+  off = p.zero_floats;
+  const int ts = tapset_floats(p.K, 2);
+  p.wlen = ts * (p.has_base + 4 * d);
+  p.wbeg = p.has_base ? 0 : ts * (1 + 4 * p.lvl0);
+  p.wchan = p.G == 1 ? p.wlen : (int)pad(p.wlen, 16);
+  p.woff = (int)off;
+  off += (long long)p.G * p.wchan;
+  p.inv_rows = 1.f / (float)(p.tiled ? 4 * p.tyn[1] + 2 * HS : h1);
+  p.inv_txn = 1.f / (float)p.txn[1];
+  for (int j = 0; j <= d; ++j) p.inv_h[j] = 1.f / (float)p.h[j];
+  p.tileoff = (int)off;
+  p.ntiles = 0;
+  for (int j = 2; j <= d; ++j) p.ntiles += p.tyn[j] * p.txn[j];
+  off += 8LL * p.ntiles + 4;              // and the barrier behind them
+  p.smem_bytes = (int)(off * 4 > (1LL << 30) ? (1LL << 30) : off * 4);
+  p.total = (long long)p.B * p.nty * p.ntx * p.ngroups;
+  // warps per CTA: the most on an SM (registers and shared memory), weighted with the share of them that has
+  // work in the rounds of the top level and with the CTAs there are
+  const int gp = imin(p.G, 8), tpw = 8 / gp;
+  const int slots = (p.G / gp) * cdiv(p.tyn[1] * p.txn[1], tpw);
+  int best = 2;
+  p.score = 0.0;
+  for (int nw = kPlanarMaxThreads / 32; nw >= 2; --nw) {
+    p.nthreads = 32 * nw;
+    const double per_sm = (double)p.total / 148.0, resident = planar_resident(p);
+    const double lanes = (double)p.G * p.tyn[1] * p.txn[1] / (8.0 * slots);    // of a warp's eight tile slots
+    const double c = (resident < per_sm ? resident : per_sm) * nw * lanes * slots / ((double)cdiv(slots, nw) * nw);
+    if (c > p.score * 1.0001) { p.score = c; best = nw; }
+  }
+  p.nthreads = 32 * best;
+  return off * 4;
+}
+
+// Persistent grid; a multiple of the channel groups keeps a CTA on one group, so that its tap sets are
+// loaded once (taken when it costs less than an eighth of the chip)
+inline void planar_grid(PlanarStage& p) {
+  const long long most = 148LL * planar_resident(p);
+  long long g = p.total < most ? p.total : most;
+  const long long whole = g / p.ngroups * p.ngroups;
+  if (p.total > g && whole * 8 >= g * 7) g = whole;
+  p.grid = (int)g;
+}
+
+// in_dtype / out type: a stage with the base path reads and writes the layer's type (0 fp32, 1 bf16, 2 fp16);
+// one without reads a plane set of `in_dtype` and writes fp32 planes
+cudaError_t launch_planar(const PlanarStage& p, int in_dtype, const void* x, void* out, const float* rin,
+                          const float* packed, cudaStream_t stream);
+
+// Low-pass planes (sums over 2^k x 2^k blocks, fp32) one to three levels below a plane set, one pass.
+struct PlanarLowpass {
+  int B, C, H, W, cl;                     // cl: lanes over channels, outputs (B, h, w, C); else (B, C, h, w)
+  long long xs[4];
+  long long off[3];                       // floats into the scratch, -1: not wanted
+  long long total;
+};
+cudaError_t launch_planar_lowpass(const PlanarLowpass& p, int in_dtype, const void* x, float* scratch, cudaStream_t stream);
+
+}  // namespace wt
