@@ -169,6 +169,18 @@ int wtconv2d_weight_grad_stats(const void* x, const void* gy, const float* x_pyr
                                const long long* x_strides, const long long* g_strides, void* stream);
 
 /*
+ * The two calls above as one: the same sums, without the pyramids in memory for kernel sizes 3, 5 and 7 (only
+ * the low-pass planes of both tensors leave the chip, a quarter of the elements per level).  g_strides are
+ * those of the output gradient at full resolution; workspace is
+ * wtconv2d_weight_grad_workspace_bytes() bytes of device scratch (16-byte aligned) or NULL if 0.
+ */
+int wtconv2d_weight_grad_workspace_bytes(int B, int C, int H, int W, int K, int L, int dtype, const long long* x_strides,
+                                         const long long* g_strides, size_t* bytes);
+int wtconv2d_weight_grad(const void* x, const void* gy, float* stats, void* workspace, size_t workspace_bytes, int B,
+                         int C, int H, int W, int K, int L, int dtype, const long long* x_strides,
+                         const long long* g_strides, void* stream);
+
+/*
  * Scratch bytes wtconv2d_forward needs for this problem and memory layout (0
  * when the whole cascade of a plane is fused on chip, which is the case for
  * small planes; larger planes hand the reconstruction of their deep levels --

@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
     (2, 3, 897, 5, 5, 1, torch.float32), (1, 2, 31, 5, 7, 1, torch.float32), (3, 5, 4097, 5, 3, 2, torch.float32),
     (2, 3, 448, 4, 5, 2, torch.float32), (2, 3, 449, 4, 7, 4, torch.float32), (1, 1, 17, 2, 5, 8, torch.float32),
     (3, 2, 1000, 3, 7, 3, torch.float32), (40, 9, 130, 0, 5, 1, torch.float32), (2, 4, 2048, 5, 5, 2, torch.bfloat16),
-    (5, 700, 64, 1, 1, 1, torch.float16),
+    (5, 700, 64, 1, 1, 1, torch.float16), (3, 3, 961, 4, 5, 1, torch.bfloat16), (4, 3, 3333, 5, 7, 1, torch.float16),
+    (2, 5, 1922, 3, 5, 1, torch.bfloat16), (3, 3, 449, 1, 7, 1, torch.bfloat16),
 ])
 def test_forward_and_gradients(B, C, N, L, K, stride, dtype):
     if not torch.cuda.is_available():

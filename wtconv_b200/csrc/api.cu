@@ -10,6 +10,8 @@
 #include "../../include/wtconv_b200.h"
 #include "wt1d_host.h"
 #include "wt1d_warp.cuh"
+#include "wt2d_corr_args.h"
+#include "wt2d_corr_host.h"
 #include "wt2d_host.h"
 #include "wt2d_wgrad.cuh"
 #include "wt_aux.h"
@@ -91,8 +93,9 @@ int make_layer2d(Layer2d& ly, const void* x, const void* y, int B, int C, int H,
 
 // Launch chains are pure functions of the layer description; the last few are kept so that a
 // model that calls the same layers step after step does not re-plan them.
-std::shared_ptr<const Chain2d> cached_chain(const Layer2d& ly) {
-  struct Entry { Layer2d key; std::shared_ptr<const Chain2d> chain; };
+template <typename Chain, Chain (*Make)(const Layer2d&)>
+std::shared_ptr<const Chain> cached_plan(const Layer2d& ly) {
+  struct Entry { Layer2d key; std::shared_ptr<const Chain> chain; };
   static std::mutex mu;
   static std::vector<Entry> entries;
   static size_t next = 0;
@@ -107,12 +110,16 @@ std::shared_ptr<const Chain2d> cached_chain(const Layer2d& ly) {
     for (const Entry& e : entries)
       if (memcmp(&e.key, &key, sizeof(key)) == 0) return e.chain;
   }
-  auto chain = std::make_shared<const Chain2d>(plan_layer(ly));
+  auto chain = std::make_shared<const Chain>(Make(ly));
   std::lock_guard<std::mutex> lock(mu);
   if (entries.size() < kCapacity) entries.push_back({key, chain});
   else { entries[next] = {key, chain}; next = (next + 1) % kCapacity; }
   return chain;
 }
+
+Chain2d make_chain(const Layer2d& ly) { return plan_layer(ly); }
+std::shared_ptr<const Chain2d> cached_chain(const Layer2d& ly) { return cached_plan<Chain2d, make_chain>(ly); }
+std::shared_ptr<const CorrChain> cached_corr(const Layer2d& ly) { return cached_plan<CorrChain, plan_corr>(ly); }
 
 }  // namespace
 
@@ -284,6 +291,67 @@ int wtconv2d_weight_grad_stats(const void* x, const void* gy, const float* x_pyr
                      per_set, cs);
     if (e != cudaSuccess) return (int)e;
     off += (size_t)B * h * w * 4 * C;
+  }
+  return WTCONV_OK;
+}
+
+// Planar correlation kernels: the unrolled sizes with a halo, on planes of more than one row (a one-row image
+// would fill a quarter of every tile)
+static bool corr_supported(int K, int H) { return (K == 3 || K == 5 || K == 7) && H > 1; }
+
+int wtconv2d_weight_grad_workspace_bytes(int B, int C, int H, int W, int K, int L, int dtype, const long long* x_strides,
+                                         const long long* g_strides, size_t* bytes) {
+  if (!bytes) return WTCONV_ERR_BAD_ARG;
+  Layer2d ly;
+  const int st = make_layer2d(ly, nullptr, nullptr, B, C, H, W, K, L, 1, dtype, x_strides, g_strides);
+  if (st) return st;
+  if (!unrolled_k(K)) return WTCONV_ERR_BAD_KERNEL_SIZE;
+  if (!corr_supported(K, H)) {
+    *bytes = 2 * wtconv2d_pyramid_floats(B, C, H, W, L) * sizeof(float);
+    return WTCONV_OK;
+  }
+  ly.x_align = ly.y_align = 16;                            // the scratch does not depend on the alignment
+  const std::shared_ptr<const CorrChain> ch = cached_corr(ly);
+  if (ch->status) return ch->status;
+  *bytes = (size_t)ch->scratch_floats * sizeof(float);
+  return WTCONV_OK;
+}
+
+int wtconv2d_weight_grad(const void* x, const void* gy, float* stats, void* workspace, size_t workspace_bytes, int B, int C, int H,
+                         int W, int K, int L, int dtype, const long long* x_strides, const long long* g_strides, void* stream) {
+  if (!x || !gy || !stats) return WTCONV_ERR_BAD_ARG;
+  size_t need = 0;
+  const int rq = wtconv2d_weight_grad_workspace_bytes(B, C, H, W, K, L, dtype, x_strides, g_strides, &need);
+  if (rq) return rq;
+  float* ws = static_cast<float*>(workspace);
+  if (need && (!ws || workspace_bytes < need)) return WTCONV_ERR_WORKSPACE;
+  if (need && ptr_align(ws) < 16) return WTCONV_ERR_MISALIGNED;
+  if (!corr_supported(K, H)) {
+    float* gp = ws ? ws + wtconv2d_pyramid_floats(B, C, H, W, L) : nullptr;
+    int st = wtconv2d_pyramid(x, ws, B, C, H, W, L, dtype, x_strides, stream);
+    if (!st) st = wtconv2d_pyramid(gy, gp, B, C, H, W, L, dtype, g_strides, stream);
+    return st ? st : wtconv2d_weight_grad_stats(x, gy, ws, gp, stats, B, C, H, W, K, L, dtype, x_strides, g_strides, stream);
+  }
+  Layer2d ly;
+  const int st = make_layer2d(ly, x, gy, B, C, H, W, K, L, 1, dtype, x_strides, g_strides);
+  if (st) return st;
+  if (ly.x_align < ly.elem_size || ly.y_align < ly.elem_size) return WTCONV_ERR_MISALIGNED;
+  const std::shared_ptr<const CorrChain> ch = cached_corr(ly);
+  if (ch->status) return ch->status;
+  cudaStream_t cs = static_cast<cudaStream_t>(stream);
+  cudaError_t e = cudaMemsetAsync(stats, 0, wtconv2d_weight_grad_stat_floats(C, K, L) * sizeof(float), cs);
+  if (e != cudaSuccess) return (int)e;
+  for (const CorrStage& sg : ch->stages) {
+    auto planes = [&](int j) { return ((long long)B * C * sg.p.h[j] * sg.p.w[j] + 3) / 4 * 4; };
+    CorrArgs a;
+    a.stats = stats; a.C = C; a.set0 = 1 + 4 * (sg.level - 1);
+    a.llx = sg.out_off < 0 ? nullptr : ws + sg.out_off;
+    a.llg = sg.out_off < 0 ? nullptr : ws + sg.out_off + planes(1);
+    a.nsplit = sg.nsplit; a.gvec = sg.gvec;
+    const bool first = sg.in_off < 0;
+    for (int i = 0; i < 4; ++i) a.gs[i] = first ? ly.ys[i] : sg.p.xs[i];
+    e = launch_corr(sg, a, dtype, first ? x : ws + sg.in_off, first ? gy : ws + sg.in_off + planes(0), cs);
+    if (e != cudaSuccess) return (int)e;
   }
   return WTCONV_OK;
 }

@@ -316,15 +316,13 @@ void grad_stats(const LayerDesc& d, const Tensor& x, const Tensor& g, Tensor& st
   long long xs[4], gs[4];
   strides(x, xs);
   strides(g, gs);
-  cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
-  const int64_t n = std::max<int64_t>((int64_t)wtconv2d_pyramid_floats(B, C, H, W, L), 1);
-  Tensor xp = at::detail::empty_cuda({n}, at::kFloat, x.device(), std::nullopt);
-  Tensor gp = at::detail::empty_cuda({n}, at::kFloat, x.device(), std::nullopt);
-  check(wtconv2d_pyramid(x.const_data_ptr(), xp.data_ptr<float>(), B, C, H, W, L, code, xs, stream), "wtconv2d_pyramid");
-  check(wtconv2d_pyramid(g.const_data_ptr(), gp.data_ptr<float>(), B, C, H, W, L, code, gs, stream), "wtconv2d_pyramid");
-  check(wtconv2d_weight_grad_stats(x.const_data_ptr(), g.const_data_ptr(), xp.data_ptr<float>(), gp.data_ptr<float>(),
-                                   stats.data_ptr<float>(), B, C, H, W, K, L, code, xs, gs, stream),
-        "wtconv2d_weight_grad_stats");
+  size_t bytes = 0;
+  check(wtconv2d_weight_grad_workspace_bytes(B, C, H, W, K, L, code, xs, gs, &bytes), "wtconv2d_weight_grad_workspace_bytes");
+  c10::DataPtr ws;
+  if (bytes) ws = c10::cuda::CUDACachingAllocator::get()->allocate(bytes);
+  check(wtconv2d_weight_grad(x.const_data_ptr(), g.const_data_ptr(), stats.data_ptr<float>(), ws.get(), bytes, B, C, H, W, K, L, code,
+                             xs, gs, c10::cuda::getCurrentCUDAStream(x.device().index()).stream()),
+        "wtconv2d_weight_grad");
 }
 
 // Gradients of all parameters from the correlation sums

@@ -20,17 +20,17 @@ cudaError_t launch_spt(Warp1dArgs a, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-// Samples per thread: 32 halve the shuffles and the neighbour-only lanes per sample, but a warp then spans
-// about 960 samples; with fewer than eight such warps per SM (or rows shorter than half a warp) 16
-// samples keep more of the chip busy.  Up to two levels the neighbour lanes are one per side either way.
+// Samples per thread: 32 halve the shuffles, the neighbour-only lanes and the per-item work per sample, but a
+// warp then spans about 960 samples; with fewer than eight such warps per SM (or rows shorter than half
+// a warp) 16 samples keep more of the chip busy.
 template <typename T, int K, int L>
 cudaError_t launch_one(const Warp1dArgs& a, cudaStream_t stream) {
   if constexpr (L == 5) return launch_spt<T, K, L, 32>(a, stream);
-  else if constexpr (L >= 3) {
+  else {
     const long long warps = (long long)a.B * a.C * cdiv(a.N, warp1d_segment(K, L, 32));
     if (a.N >= 480 && warps >= 148 * 8) return launch_spt<T, K, L, 32>(a, stream);
     return launch_spt<T, K, L, 16>(a, stream);
-  } else return launch_spt<T, K, L, 16>(a, stream);
+  }
 }
 
 template <typename T, int K, int L>

@@ -109,6 +109,24 @@ __device__ __forceinline__ void warp1d_copy16(void* dst, const void* src, int by
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
 }
 
+// Rows that do not start on a 16-byte boundary: a stream of aligned words of WB bytes from `base`, `late` elements
+// before the row; bytes past the row arrive as zeros.  (Not unrolled whole: the copy appears twice in a kernel
+// and the code must fit the instruction cache.)
+template <typename T, int SPT, int WB>
+__device__ __forceinline__ void warp1d_stream(const T* __restrict__ base, int late, int tw, int lane, int N, unsigned char* st) {
+  constexpr int CPT = SPT * (int)sizeof(T) / 16;
+  constexpr int EPW = WB / (int)sizeof(T), WPC = 16 / WB;           // elements per word, words per chunk
+#pragma unroll 8
+  for (int k = 0; k < SPT / EPW; ++k) {
+    const int word = lane + 32 * k, t = tw + word * EPW;            // element of `base`
+    const int left = (N + late - t) * (int)sizeof(T);               // bytes up to the end of the row
+    const int n = (t >= 0 && left > 0) ? imin(left, WB) : 0;
+    unsigned char* d = st + warp1d_own<T, SPT>(word / (WPC * CPT), (word / WPC) & (CPT - 1)) + (word & (WPC - 1)) * WB;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((unsigned)__cvta_generic_to_shared(d)),
+                 "l"(n ? base + t : base), "n"(WB), "r"(n) : "memory");
+  }
+}
+
 // Starts the copy of samples tw .. tw + 32 * SPT - 1 of a row of N samples (zeros outside) into the staging
 // buffer; complete after cp.async wait and __syncwarp.  up > 1: the row holds N / up values and sample t is
 // row[t / up] / up.
@@ -128,29 +146,52 @@ __device__ __forceinline__ void warp1d_fetch(const T* __restrict__ xr, int tw, i
         warp1d_copy16(st + warp1d_line<T, SPT>(lane, k), n ? p + 32 * VEC * k : xr, n);
       }
     }
+  } else if (up == 1 && (reinterpret_cast<uintptr_t>(xr) & 7) == 0) {
+    warp1d_stream<T, SPT, 8>(xr, 0, tw, lane, N, st);
+  } else if (up == 1) {
+    // A 16-bit row that starts in the middle of a word is staged one element late (warp1d_read shifts it back)
+    const int late = (int)((reinterpret_cast<uintptr_t>(xr) & 3) / sizeof(T));
+    warp1d_stream<T, SPT, 4>(xr - late, late, tw, lane, N, st);
+    if (sizeof(T) == 2 && lane == 0) {                              // the word behind the last run
+      const int t = tw + 32 * SPT, left = (N + late - t) * (int)sizeof(T);
+      const int n = (late && t >= 0 && left > 0) ? imin(left, 4) : 0;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(st + 32 * SPT * sizeof(T))),
+                   "l"(n ? xr - late + t : xr - late), "r"(n) : "memory");
+    }
   } else {
     const unsigned limit = (unsigned)(N / up * up);
     const float inv = 1.f / (float)up;
-#pragma unroll 8                                                    // not whole: the loop appears twice and the code must fit the instruction cache
+#pragma unroll 8
     for (int k = 0; k < SPT; ++k) {
       const int idx = lane + 32 * k;
       const unsigned t = (unsigned)(tw + idx);                      // negative positions wrap beyond the limit
       T* d = reinterpret_cast<T*>(st + warp1d_own<T, SPT>(idx / SPT, (idx / VEC) & (CPT - 1))) + (idx & (VEC - 1));
-      if (sizeof(T) == 4 && up == 1) {
-        async_copy4_zfill(d, t < limit ? xr + t : xr, t < limit);
-      } else {
-        float v = 0.f;
-        if (t < limit) v = up == 1 ? Elem<T>::to_f(xr[t]) : Elem<T>::to_f(xr[t / (unsigned)up]) * inv;
-        *d = Elem<T>::from_f(v);
-      }
+      *d = Elem<T>::from_f(t < limit ? Elem<T>::to_f(xr[t / (unsigned)up]) * inv : 0.f);
     }
   }
 }
 
-// This thread's run
+// This thread's run, which starts at sample tw + lane * SPT; late: in the middle of its first word (16-bit types)
 template <typename T, int SPT>
-__device__ __forceinline__ void warp1d_read(const unsigned char* st, int lane, float (&v)[SPT]) {
+__device__ __forceinline__ void warp1d_read(const unsigned char* st, int lane, int tw, bool late, float (&v)[SPT]) {
   constexpr int VEC = 16 / (int)sizeof(T), CPT = SPT / VEC;
+  if (sizeof(T) == 2 && late) {
+    unsigned w[4 * CPT + 1];
+#pragma unroll
+    for (int k = 0; k < CPT; ++k) {
+      const uint4 q = *reinterpret_cast<const uint4*>(st + warp1d_own<T, SPT>(lane, k));
+      w[4 * k] = q.x; w[4 * k + 1] = q.y; w[4 * k + 2] = q.z; w[4 * k + 3] = q.w;
+    }
+    w[4 * CPT] = *reinterpret_cast<const unsigned*>(lane == 31 ? st + 32 * SPT * sizeof(T) : st + warp1d_own<T, SPT>(lane + 1, 0));
+#pragma unroll
+    for (int k = 0; k < 4 * CPT; ++k) {
+      Chunk<T, 4> ch;
+      ch.raw = __funnelshift_r(w[k], w[k + 1], 16);
+      v[(2 * k) % SPT] = Elem<T>::to_f(ch.get(0)); v[(2 * k + 1) % SPT] = Elem<T>::to_f(ch.get(1 % ch.VEC));
+    }
+    if (tw + (lane + 1) * SPT == 0) v[SPT - 1] = 0.f;              // the row's first word also holds the element before it
+    return;
+  }
 #pragma unroll
   for (int k = 0; k < CPT; ++k) {
     Chunk<T, 16> ch;
@@ -192,7 +233,7 @@ struct Warp1dLevel {
 
 // Dynamic shared memory: per warp two staging buffers and two tap-set buffers
 template <typename T, int K, int L, int SPT>
-constexpr size_t warp1d_smem_bytes() { return (size_t)kWarp1dWarps * 2 * (32 * SPT * sizeof(T) + warp1d_tap_words(K, L) * 16); }
+constexpr size_t warp1d_smem_bytes() { return (size_t)kWarp1dWarps * 2 * (32 * SPT * sizeof(T) + 16 + warp1d_tap_words(K, L) * 16); }
 
 // A warp walks over (row, segment) items and copies the samples and taps of the next one while it computes
 // the current one.  Registers: the run, the accumulated output and one level's bands are live at once
@@ -209,7 +250,7 @@ wt1d_warp_kernel(const __grid_constant__ Warp1dArgs a) {
   constexpr int VEC = 16 / (int)sizeof(T);             // samples per 128-bit access
   constexpr int CPT = SPT / VEC;                       // 128-bit accesses per thread
   constexpr int NW4 = warp1d_tap_words(K, L);
-  constexpr int BUF = 32 * SPT * (int)sizeof(T), STEP = BUF + NW4 * 16;
+  constexpr int BUF = 32 * SPT * (int)sizeof(T) + 16, STEP = BUF + NW4 * 16;   // + the word behind the last run
   extern __shared__ __align__(128) unsigned char warp1d_smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned char* const buf0 = warp1d_smem + warp * 2 * STEP;
@@ -244,7 +285,8 @@ wt1d_warp_kernel(const __grid_constant__ Warp1dArgs a) {
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncwarp();
     float xv[SPT];
-    warp1d_read<T, SPT>(st, lane, xv);
+    const T* xrow = static_cast<const T*>(a.x) + cur.n * a.xs0 + cur.c * a.xs1;
+    warp1d_read<T, SPT>(st, lane, cur.tw, a.up == 1 && (reinterpret_cast<uintptr_t>(xrow) & 3), xv);
     const float* wch = reinterpret_cast<const float*>(st + BUF);
 
     // ---- levels, deepest first (recursion), then the base convolution and the bias
@@ -312,6 +354,22 @@ wt1d_warp_kernel(const __grid_constant__ Warp1dArgs a) {
               if (t + i < a.N) yr[t + i] = ch.get(i);
           }
         }
+      } else if (sizeof(T) == 2) {
+        // word by word: elements (2i - late, 2i - late + 1) of the segment
+        const int late = (int)((reinterpret_cast<uintptr_t>(yr) & 3) / 2);
+        auto at = [&](int idx) { return *(reinterpret_cast<const T*>(st + warp1d_own<T, SPT>(idx / SPT, (idx / VEC) & (CPT - 1))) + (idx & (VEC - 1))); };
+#pragma unroll 8
+        for (int k = 0; k <= SPT / 2; ++k) {
+          const int idx = 2 * (lane + 32 * k) - late + HL * SPT, t = cur.tw + idx;
+          const bool in0 = idx >= HL * SPT && idx < (32 - HL) * SPT && t < a.N;
+          const bool in1 = idx + 1 < (32 - HL) * SPT && t + 1 < a.N;
+          if (in0 && in1) {
+            Chunk<T, 4> ch;
+            ch.set(0, at(idx)); ch.set(1 % ch.VEC, at(idx + 1));
+            *reinterpret_cast<unsigned*>(yr + t) = ch.raw;
+          } else if (in0) yr[t] = at(idx);
+          else if (in1 && idx + 1 >= HL * SPT) yr[t + 1] = at(idx + 1);
+        }
       } else {
 #pragma unroll 8
         for (int k = 0; k < SPT; ++k) {
@@ -378,7 +436,7 @@ struct Warp1dGradLevel {
 // Dynamic shared memory: two buffers of the x run and the g run per warp (the next item is copied while
 // this one is computed)
 template <typename T, int SPT>
-constexpr size_t warp1d_wgrad_smem() { return (size_t)kWarp1dWarps * 4 * 32 * SPT * sizeof(T); }
+constexpr size_t warp1d_wgrad_smem() { return (size_t)kWarp1dWarps * 4 * (32 * SPT * sizeof(T) + 16); }
 
 template <typename T, int K, int L, int SPT>
 __global__ void __launch_bounds__(kWarp1dWarps * 32, (K <= 5 && L <= 4) ? 2 : 1)
@@ -386,7 +444,7 @@ wt1d_wgrad_kernel(const __grid_constant__ Wgrad1dArgs a) {
 #ifdef __CUDA_ARCH__
   constexpr int HL = warp1d_halo(K, L, SPT), SEG = warp1d_segment(K, L, SPT);
   constexpr int NA = K + 1 + 2 * L * K;                // base taps, sum of g, then (low, high) taps per level
-  constexpr int BUF = 32 * SPT * (int)sizeof(T);
+  constexpr int BUF = 32 * SPT * (int)sizeof(T) + 16;
   extern __shared__ __align__(128) unsigned char warp1d_smem[];
   static_assert(NA * (int)sizeof(float) <= 4 * BUF, "the sums of a warp fit its buffers");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -413,8 +471,11 @@ wt1d_wgrad_kernel(const __grid_constant__ Wgrad1dArgs a) {
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncwarp();
     float xv[SPT], gv[SPT];
-    warp1d_read<T, SPT>(st + cur * 2 * BUF, lane, xv);
-    warp1d_read<T, SPT>(st + cur * 2 * BUF + BUF, lane, gv);
+    const int n = (int)(it / a.nseg), tw = (int)(it - (long long)n * a.nseg) * SEG - HL * SPT;
+    const T* xr = static_cast<const T*>(a.x) + n * a.xs0 + c * a.xs1;
+    const T* gr = static_cast<const T*>(a.g) + n * a.gs0 + c * a.gs1;
+    warp1d_read<T, SPT>(st + cur * 2 * BUF, lane, tw, reinterpret_cast<uintptr_t>(xr) & 3, xv);
+    warp1d_read<T, SPT>(st + cur * 2 * BUF + BUF, lane, tw, a.up == 1 && (reinterpret_cast<uintptr_t>(gr) & 3), gv);
 #pragma unroll
     for (int o = 0; o < SPT; ++o) {                    // the outer lanes' positions belong to the neighbouring segments
       gv[o] = owner ? gv[o] : 0.f;

@@ -442,6 +442,7 @@ inline bool plan_planar(PlanarStage& p, const Layer2d& ly, const int* Hl, const 
                         bool tiled, bool x_src, bool cl) {
   p = PlanarStage();
   p.B = ly.B; p.C = ly.C; p.K = ly.K; p.nlev = nlev; p.lvl0 = first;
+  p.ctas = planar_ctas(ly.K);
   p.has_base = final_stage ? 1 : 0;
   p.tiled = tiled ? 1 : 0;
   for (int j = 0; j <= nlev; ++j) { p.h[j] = Hl[first + j]; p.w[j] = Wl[first + j]; }

@@ -104,20 +104,27 @@ template <typename T, int VEC>
 struct PlanarQuad {
   typedef typename RawChunk<(VEC * (int)sizeof(T) < 4 ? 4 : VEC * (int)sizeof(T))>::type raw_t;
   raw_t raw[4 / VEC];
-  __device__ __forceinline__ void load(const T* __restrict__ p, int x, int W, long long step, bool ok) {
+  __device__ __forceinline__ void load(const T* __restrict__ p, int x, int W, int step, bool ok) {
+    const T* q = p + (VEC > 1 ? x : x * step);
+    if (VEC == 1 && ok && x >= 0 && x + 4 <= W) {               // the usual case: no check per pixel
+#pragma unroll
+      for (int k = 0; k < 4 / VEC; ++k) { put(k, *q); q += step; }
+      return;
+    }
 #pragma unroll
     for (int k = 0; k < 4 / VEC; ++k) {
       raw[k] = raw_t();                                         // zero bits are 0.0 in every type
       const int xx = x + k * VEC;
       if (!ok || xx < 0 || xx >= W) continue;
-      if (VEC > 1) raw[k] = __ldg(reinterpret_cast<const raw_t*>(p + xx));
-      else {
-        Chunk<T, 4> c;
-        c.raw = 0u;
-        c.set(0, p[(long long)xx * step]);
-        *reinterpret_cast<unsigned*>(&raw[k]) = c.raw;
-      }
+      if (VEC > 1) raw[k] = __ldg(reinterpret_cast<const raw_t*>(q + k * VEC));
+      else put(k, q[k * step]);
     }
+  }
+  __device__ __forceinline__ void put(int k, T v) {
+    Chunk<T, 4> c;
+    c.raw = 0u;
+    c.set(0, v);
+    *reinterpret_cast<unsigned*>(&raw[k]) = c.raw;
   }
   __device__ __forceinline__ float get(int i) const {
     Chunk<T, (VEC * (int)sizeof(T) < 4 ? 4 : VEC * (int)sizeof(T))> c;
@@ -158,23 +165,6 @@ struct PlanarFill {
   float inv_nr;                       // 1 / (rb - ra)
   static constexpr int HS = K / 2;
 
-  __device__ __forceinline__ void put_pixels(int g, int r, int dy, int c, float v0, float v1) const {
-    const int fr = 2 * r - HS + dy, fc = 2 * c - HS;
-    float* d = sm + p.xoff + g * p.xplane + fr * p.xpitch + fc;
-    if (!p.tiled) {                    // interior positions only: always inside the frame
-      if (HS % 2 == 0) *reinterpret_cast<float2*>(d) = make_float2(v0, v1);
-      else { d[0] = v0; d[1] = v1; }
-      return;
-    }
-    if (fr < 0 || fr >= p.xrows) return;
-    if (HS % 2 == 0) {
-      if (fc >= 0 && fc < p.xcols) *reinterpret_cast<float2*>(d) = make_float2(v0, v1);
-    } else {
-      if (fc >= 0 && fc < p.xcols) d[0] = v0;
-      if (fc + 1 >= 0 && fc + 1 < p.xcols) d[1] = v1;
-    }
-  }
-
   // two neighbouring cells of a frame row
   static __device__ __forceinline__ void put2(float* d, float v0, float v1) {
     if (HS % 2 == 0) *reinterpret_cast<float2*>(d) = make_float2(v0, v1);
@@ -208,7 +198,7 @@ struct PlanarFill {
         for (int k = 0; k < NR; ++k)
 #pragma unroll
           for (int h = 0; h < (1 << SHIFT); ++h)
-            q[k][h].load(src + so + k * (int)p.xs[2], x + 4 * h, W, p.xs[3], more && y + k >= 0 && y + k < H);
+            q[k][h].load(src + so + k * (int)p.xs[2], x + 4 * h, W, (int)p.xs[3], more && y + k >= 0 && y + k < H);
       };
       fetch(wk.row < nrows);
       for (int row = wk.row; row < nrows; row += wk.step) {
@@ -274,62 +264,74 @@ struct PlanarFill {
     }
   }
 
-  // channel chunks: one item = V channels of one position
+  // Channel chunks: one item = V channels of one position.  Everything that does not depend on the channel
+  // (bounds, offsets) is worked out once per item; a channel costs its conversions, the Haar step and stores
+  // at four running addresses.
   template <int CB>
   __device__ __forceinline__ void chunks(int tid, int nthr) const {
-    constexpr int V = CB / (int)sizeof(T);
+    constexpr int V = CB / (int)sizeof(T), NP = 2 << SHIFT;     // pixels per side of a position
+    typedef typename RawChunk<CB>::type raw_t;
     const int H = p.Hsrc, W = p.Wsrc;
     const int nch = p.G / V, ncols = cb - ca;
     const PlanarWalk wk(ncols, tid, nthr);
     const int nr = rb - ra, nrows = nch * nr;
+    const int s2 = (int)p.xs[2], s3 = (int)p.xs[3], splane = p.splane[1];
     for (int row = wk.row; row < nrows; row += wk.step) {
       const int ch = planar_div(row, inv_nr), r = ra + row - ch * nr;          // chunk slowest: a warp covers neighbouring pixels
-      const int y = (2 << SHIFT) * (py0 + r);
+      const int y = NP * (py0 + r);
       for (int c = ca + wk.col; c < cb; c += 32) {
-        const int x = (2 << SHIFT) * (px0 + c);
-        float v[2][2][V];
+        const int x = NP * (px0 + c);
+        Chunk<T, CB> q[NP][NP];
+        {
+          const T* q0 = src + (y * s2 + x * s3 + ch * V);
+          const bool inside = y >= 0 && x >= 0 && y + NP <= H && x + NP <= W;
 #pragma unroll
-        for (int by = 0; by < 2; ++by)
+          for (int dy = 0; dy < NP; ++dy)
 #pragma unroll
-          for (int bx = 0; bx < 2; ++bx) {
-            if (SHIFT == 0) {
-              Chunk<T, CB> q = load<CB>(y + by, x + bx, H, W, ch);
-#pragma unroll
-              for (int e = 0; e < V; ++e) v[by][bx][e] = Elem<T>::to_f(q.get(e));
-            } else {
-              const int yy = y + 2 * by, xx = x + 2 * bx;
-              const Chunk<T, CB> q0 = load<CB>(yy, xx, H, W, ch), q1 = load<CB>(yy, xx + 1, H, W, ch);
-              const Chunk<T, CB> q2 = load<CB>(yy + 1, xx, H, W, ch), q3 = load<CB>(yy + 1, xx + 1, H, W, ch);
-#pragma unroll
-              for (int e = 0; e < V; ++e)
-                v[by][bx][e] = (Elem<T>::to_f(q0.get(e)) + Elem<T>::to_f(q1.get(e))) + (Elem<T>::to_f(q2.get(e)) + Elem<T>::to_f(q3.get(e)));
+            for (int dx = 0; dx < NP; ++dx) {
+              q[dy][dx].raw = raw_t();                          // zero bits are 0.0 in every type
+              if (inside || (y + dy >= 0 && y + dy < H && x + dx >= 0 && x + dx < W))
+                q[dy][dx].raw = __ldg(reinterpret_cast<const raw_t*>(q0 + dy * s2 + dx * s3));
             }
-          }
+        }
+        const int fr = 2 * r - HS, fc = 2 * c - HS;             // first pixel in the pixel frame
+        const bool c0 = FINAL && fc >= 0 && fc < p.xcols, c1 = FINAL && fc + 1 >= 0 && fc + 1 < p.xcols;
+        const bool r0 = fr >= 0 && fr < p.xrows, r1 = fr + 1 >= 0 && fr + 1 < p.xrows;
+        const bool pair = c0 && c1;
+        float* xd = sm + p.xoff + ch * V * p.xplane + fr * p.xpitch + fc;
+        float* sd = sm + p.soff[1] + 4 * ch * V * splane + r * p.spitch[1] + c;
 #pragma unroll
         for (int e = 0; e < V; ++e) {
-          const int g = ch * V + e;
-          const float a = v[0][0][e], b = v[0][1][e], cc = v[1][0][e], d = v[1][1][e];
-          if (FINAL) { put_pixels(g, r, 0, c, a, b); put_pixels(g, r, 1, c, cc, d); }
-          if (p.nlev > 0) {
-            float s[4];
-            planar_haar(a, b, cc, d, s);
-            float* o = sm + p.soff[1] + (4 * g) * p.splane[1] + r * p.spitch[1] + c;
+          float v[2][2];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) o[k * p.splane[1]] = s[k];
+          for (int k = 0; k < 4; ++k) {
+            const int by = k >> 1, bx = k & 1;
+            if (SHIFT == 0) v[by][bx] = Elem<T>::to_f(q[by][bx].get(e));
+            else {
+              const int yy = (2 * by) % NP, xx = (2 * bx) % NP;
+              v[by][bx] = (Elem<T>::to_f(q[yy][xx].get(e)) + Elem<T>::to_f(q[yy][(xx + 1) % NP].get(e))) +
+                          (Elem<T>::to_f(q[(yy + 1) % NP][xx].get(e)) + Elem<T>::to_f(q[(yy + 1) % NP][(xx + 1) % NP].get(e)));
+            }
+          }
+          if (FINAL) {
+            if (pair) {
+              if (r0) put2(xd, v[0][0], v[0][1]);
+              if (r1) put2(xd + p.xpitch, v[1][0], v[1][1]);
+            } else if (HS % 2) {                                // an odd halo splits the outermost positions
+              if (r0) { if (c0) xd[0] = v[0][0]; if (c1) xd[1] = v[0][1]; }
+              if (r1) { if (c0) xd[p.xpitch] = v[1][0]; if (c1) xd[p.xpitch + 1] = v[1][1]; }
+            }
+            xd += p.xplane;
+          }
+          if (p.nlev > 0) {
+            float b[4];
+            planar_haar(v[0][0], v[0][1], v[1][0], v[1][1], b);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) { sd[0] = b[k]; sd += splane; }
           }
         }
       }
     }
-  }
-
-  template <int CB>
-  __device__ __forceinline__ Chunk<T, CB> load(int y, int x, int H, int W, int ch) const {
-    typedef typename RawChunk<CB>::type raw_t;
-    Chunk<T, CB> q;
-    q.raw = raw_t();                                            // zero bits are 0.0 in every type
-    if (y >= 0 && y < H && x >= 0 && x < W)
-      q.raw = __ldg(reinterpret_cast<const raw_t*>(src + (long long)y * p.xs[2] + (long long)x * p.xs[3] + ch * (CB / (int)sizeof(T))));
-    return q;
   }
 
   __device__ __forceinline__ void run(int tid, int nthr) const {

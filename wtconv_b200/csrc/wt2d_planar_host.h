@@ -32,6 +32,8 @@ struct PlanarStage {
   int tileoff, ntiles;                    // descriptors of the tiles below the top level
   int shift, Hsrc, Wsrc;                  // 1: plane 0 is the 2 x 2 block sums of the Hsrc x Wsrc tensor read (else plane 0 itself)
   int nthreads, smem_bytes, grid;
+  int ctas;                               // CTAs of 256 threads per SM the kernel's registers allow
+  int frames_only;                        // 1: no reconstructions, tap sets or tile table (parameter gradients)
   double score;                           // planner's estimate of the busy warps per SM
   long long total;                        // work items: samples x tiles x channel groups
   long long xs[4], ys[4], rs[4];          // element strides (n, c, row, col): input, output, deeper reconstruction
@@ -40,7 +42,7 @@ struct PlanarStage {
 };
 
 inline int planar_resident(const PlanarStage& p) {          // CTAs per SM
-  const int by_smem = (228 * 1024) / (p.smem_bytes + 1024), by_regs = planar_ctas(p.K) * kPlanarMaxThreads / p.nthreads;
+  const int by_smem = (228 * 1024) / (p.smem_bytes + 1024), by_regs = p.ctas * kPlanarMaxThreads / p.nthreads;
   return imax(1, imin(by_smem, by_regs));
 }
 
@@ -82,7 +84,7 @@ inline long long planar_layout(PlanarStage& p) {
   if (p.has_base) off += (long long)p.G * p.xplane;
   p.jlocal = d + 1;
   for (int j = d; j >= 2 && p.h[j] * p.w[j] <= 64; --j) p.jlocal = j;
-  for (int j = 1; j < d; ++j) {
+  for (int j = 1; j < d && !p.frames_only; ++j) {
     const int cols = 8 * p.txn[j + 1];
     p.epitch[j] = cols + 4;
     p.eplane[j] = (int)pad((long long)8 * p.tyn[j + 1] * p.epitch[j], 8);
@@ -92,7 +94,7 @@ inline long long planar_layout(PlanarStage& p) {
   p.zero_floats = (int)((off + 3) / 4 * 4);
   off = p.zero_floats;
   const int ts = tapset_floats(p.K, 2);
-  p.wlen = ts * (p.has_base + 4 * d);
+  p.wlen = p.frames_only ? 0 : ts * (p.has_base + 4 * d);
   p.wbeg = p.has_base ? 0 : ts * (1 + 4 * p.lvl0);
   p.wchan = p.G == 1 ? p.wlen : (int)pad(p.wlen, 16);
   p.woff = (int)off;
@@ -102,7 +104,7 @@ inline long long planar_layout(PlanarStage& p) {
   for (int j = 0; j <= d; ++j) p.inv_h[j] = 1.f / (float)p.h[j];
   p.tileoff = (int)off;
   p.ntiles = 0;
-  for (int j = 2; j <= d; ++j) p.ntiles += p.tyn[j] * p.txn[j];
+  for (int j = 2; j <= d && !p.frames_only; ++j) p.ntiles += p.tyn[j] * p.txn[j];
   off += 8LL * p.ntiles + 4;              // and the barrier behind them
   p.smem_bytes = (int)(off * 4 > (1LL << 30) ? (1LL << 30) : off * 4);
   p.total = (long long)p.B * p.nty * p.ntx * p.ngroups;
@@ -110,14 +112,18 @@ inline long long planar_layout(PlanarStage& p) {
   // work in the rounds of the top level and with the CTAs there are
   const int gp = imin(p.G, 8), tpw = 8 / gp;
   const int slots = (p.G / gp) * cdiv(p.tyn[1] * p.txn[1], tpw);
-  int best = 2;
+  int best = 2, warps = 0;
   p.score = 0.0;
   for (int nw = kPlanarMaxThreads / 32; nw >= 2; --nw) {
     p.nthreads = 32 * nw;
-    const double per_sm = (double)p.total / 148.0, resident = planar_resident(p);
+    const int resident = planar_resident(p);
+    const double per_sm = (double)p.total / 148.0;
     const double lanes = (double)p.G * p.tyn[1] * p.txn[1] / (8.0 * slots);    // of a warp's eight tile slots
     const double c = (resident < per_sm ? resident : per_sm) * nw * lanes * slots / ((double)cdiv(slots, nw) * nw);
-    if (c > p.score * 1.0001) { p.score = c; best = nw; }
+    // of equal choices the one with more warps on an SM (they also load and transform), then smaller CTAs
+    // (their barrier phases overlap with one another's work), down to four warps
+    const bool better = c > p.score * 1.0001, equal = c > p.score * 0.9999;
+    if (better || (equal && nw >= 4 && resident * nw >= warps)) { p.score = c; best = nw; warps = resident * nw; }
   }
   p.nthreads = 32 * best;
   return off * 4;
