@@ -30,13 +30,13 @@ inline int ptr_align(const void* p) {
   return al;
 }
 
+// The CTA-tile kernels: K = 1, unaligned channels-last tensors with K = 5, and the run-time size for the rest
+// (the planar kernels take 3, 5 and 7 elsewhere)
 cudaError_t launch_wt2d(const Plan2d& p, int dtype, const void* x, void* y, const float* packed, const float* rin,
                         float* rout, size_t smem, cudaStream_t st) {
   switch (p.K) {
     case 1: return launch_wt2d_k<1>(p, dtype, x, y, packed, rin, rout, smem, st);
-    case 3: return launch_wt2d_k<3>(p, dtype, x, y, packed, rin, rout, smem, st);
     case 5: return launch_wt2d_k<5>(p, dtype, x, y, packed, rin, rout, smem, st);
-    case 7: return launch_wt2d_k<7>(p, dtype, x, y, packed, rin, rout, smem, st);
     default: return launch_wt2d_k<0>(p, dtype, x, y, packed, rin, rout, smem, st);
   }
 }

@@ -208,30 +208,51 @@ cudaError_t launch_cl_pyramid(int dtype, const void* x, const long long* xs, int
   }
 }
 
+namespace {
+
+template <int K>
+cudaError_t launch_deep_k(const ClDeepArgs& a, int dtype, const void* s2, const float* packed, float* rout, int* status, cudaStream_t st) {
+  switch (dtype) {
+    case 0: return launch_deep_t<float, K>(a, s2, packed, rout, status, st);
+    case 1: return launch_deep_t<__nv_bfloat16, K>(a, s2, packed, rout, status, st);
+    default: return launch_deep_t<__half, K>(a, s2, packed, rout, status, st);
+  }
+}
+
+template <int K>
+cudaError_t launch_level_k(const ClStage& s, int dtype, const void* x, const float* rin, void* out, const float* packed, int* status,
+                           cudaStream_t st) {
+  if (s.has_base) {
+    switch (dtype) {
+      case 0: return launch_shape<float, float, K, true>(s, x, rin, out, packed, status, st);
+      case 1: return launch_shape<__nv_bfloat16, __nv_bfloat16, K, true>(s, x, rin, out, packed, status, st);
+      default: return launch_shape<__half, __half, K, true>(s, x, rin, out, packed, status, st);
+    }
+  }
+  switch (dtype) {
+    case 0: return launch_shape<float, float, K, false>(s, x, rin, out, packed, status, st);
+    case 1: return launch_shape<__nv_bfloat16, float, K, false>(s, x, rin, out, packed, status, st);
+    default: return launch_shape<__half, float, K, false>(s, x, rin, out, packed, status, st);
+  }
+}
+
+}  // namespace
+
 cudaError_t launch_cl_deep(const ClDeepArgs& a, int K, int dtype, const void* s2, const float* packed, float* rout,
                            int* status, cudaStream_t st) {
-  if (K != 5) return cudaErrorNotSupported;
-  switch (dtype) {
-    case 0: return launch_deep_t<float, 5>(a, s2, packed, rout, status, st);
-    case 1: return launch_deep_t<__nv_bfloat16, 5>(a, s2, packed, rout, status, st);
-    default: return launch_deep_t<__half, 5>(a, s2, packed, rout, status, st);
+  switch (K) {
+    case 3: return launch_deep_k<3>(a, dtype, s2, packed, rout, status, st);
+    case 5: return launch_deep_k<5>(a, dtype, s2, packed, rout, status, st);
+    default: return cudaErrorNotSupported;
   }
 }
 
 cudaError_t launch_cl_level(const ClStage& s, int dtype, const void* x, const float* rin, void* out,
                             const float* packed, int* status, cudaStream_t st) {
-  if (s.K != 5) return cudaErrorNotSupported;
-  if (s.has_base) {
-    switch (dtype) {
-      case 0: return launch_shape<float, float, 5, true>(s, x, rin, out, packed, status, st);
-      case 1: return launch_shape<__nv_bfloat16, __nv_bfloat16, 5, true>(s, x, rin, out, packed, status, st);
-      default: return launch_shape<__half, __half, 5, true>(s, x, rin, out, packed, status, st);
-    }
-  }
-  switch (dtype) {
-    case 0: return launch_shape<float, float, 5, false>(s, x, rin, out, packed, status, st);
-    case 1: return launch_shape<__nv_bfloat16, float, 5, false>(s, x, rin, out, packed, status, st);
-    default: return launch_shape<__half, float, 5, false>(s, x, rin, out, packed, status, st);
+  switch (s.K) {
+    case 3: return launch_level_k<3>(s, dtype, x, rin, out, packed, status, st);
+    case 5: return launch_level_k<5>(s, dtype, x, rin, out, packed, status, st);
+    default: return cudaErrorNotSupported;
   }
 }
 

@@ -1,6 +1,6 @@
 // Channels-last level stage of the 2-D WTConv forward for sm_100a.
 //
-// One launch computes one wavelet level of wtconv/wtconv2d.py:46-78 on a channels-last
+// One launch (K = 3 or 5) computes one wavelet level of wtconv/wtconv2d.py:46-78 on a channels-last
 // plane set, optionally together with the base path of :81-82:
 //
 //   out = IWT( conv_s(WT(in)) * scale_s  +  [LL slot: reconstruction of the deeper levels] )
@@ -868,9 +868,13 @@ __global__ void __launch_bounds__(256) wt2d_cl_lowpass4_kernel(const __grid_cons
 // (16-bit) or 256-byte (fp32) line per position, and the synthesis butterfly
 // (wavelet.py:70-75) is two xor-shuffles across the sub-band bits of the lane index.
 // ---------------------------------------------------------------------------
-constexpr int kClDeepSetPitch = (5 * 5 + 1) * kClGroup * 4 + 64;   // bytes between the staged tap sets of a level (K = 5):
-                                                                  // 64 past a multiple of 128, so the two sets read by a half warp (64 bytes each) fall into different banks
-constexpr int kClDeepLevelBytes = (4 * kClDeepSetPitch + 127) / 128 * 128;
+// Bytes between the staged tap sets of a level: 64 past a multiple of 128, so the two sets read by a half warp
+// (64 bytes each) fall into different banks
+template <int K> struct ClDeepTaps {
+  static constexpr int set_pitch = (K * K + 1) * kClGroup * 4 + 64;
+  static constexpr int level_bytes = (4 * set_pitch + 127) / 128 * 128;
+  static_assert(set_pitch % 128 == 64, "an even number of taps and the bias slot");
+};
 
 #ifdef __CUDA_ARCH__
 // Sub-band convolutions + synthesis of level j for every tile of the CTA's slots.
@@ -891,7 +895,7 @@ __device__ __forceinline__ void cl_deep_level(const ClDeepArgs& a, int j, unsign
   // taps of this lane's sub-band and channel pair: once per level
   float2 wr[K * K];
   {
-    const float2* w = reinterpret_cast<const float2*>(wlev + sbi * kClDeepSetPitch) + cp;
+    const float2* w = reinterpret_cast<const float2*>(wlev + sbi * ClDeepTaps<K>::set_pitch) + cp;
 #pragma unroll
     for (int t = 0; t < K * K; ++t) wr[t] = w[t * kClLanes];
   }
@@ -985,7 +989,7 @@ template <typename T, int K>
 __global__ void __launch_bounds__(kClDeepThreads, 2)
 wt2d_cl_deep_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ ClDeepArgs a) {
 #ifdef __CUDA_ARCH__
-  static_assert(K == 5, "the staged tap sets are laid out for K = 5");
+  constexpr int kClDeepSetPitch = ClDeepTaps<K>::set_pitch, kClDeepLevelBytes = ClDeepTaps<K>::level_bytes;
   constexpr int HS = K / 2;
   constexpr int TAPS = K * K + 1;
   constexpr int POS = 4 * kClGroup;

@@ -368,7 +368,7 @@ inline bool plan_whole_plane(Plan2d& p, long long& smem, bool& good, const Layer
 // The channels-last kernels (wt2d_cl.cuh) read the layer input through a tensor map: channel
 // stride 1, every other stride and the base address multiples of 16 bytes.
 inline bool cl_stage_supported(const Layer2d& ly) {
-  if (ly.K != 5 || ly.stride != 1 || ly.C < 8) return false;
+  if ((ly.K != 5 && ly.K != 3) || ly.stride != 1 || ly.C < 8) return false;
   if ((long long)ly.B * ly.C * ly.H * ly.W >= (1LL << 35)) return false;   // 32-bit item indices in the pyramid kernels
   if (ly.xs[1] != 1 || ly.ys[1] != 1) return false;
   if (ly.x_align < 16) return false;
@@ -605,6 +605,30 @@ inline Chain2d plan_layer(const Layer2d& ly, const Tuning2d& tune = Tuning2d()) 
   Hl[0] = ly.H; Wl[0] = ly.W;
   for (int j = 1; j <= ly.L; ++j) { Hl[j] = (Hl[j - 1] + 1) / 2; Wl[j] = (Wl[j - 1] + 1) / 2; }
 
+  // Channels-last tensors too small to fill the chip: one launch of the planar kernel with every level on chip
+  // instead of the three of the chains below, whose launches and hand-overs are then most of the time.  Measured
+  // (K = 5, bf16): 1x384x14x14 9 against 21 us, 16x384x14x14 (1.2 M elements) 19 against 25, 4x192x28x28 14 against 17,
+  // 16x192x28x28 (2.4 M) 31 against 30; planes above 32 x 32 leave fewer of them on an SM: 1x96x56x56 (0.3 M) 15
+  // against 24, 4x96x56x56 (1.2 M) 29 against 24.  Small planes without a register-level kernel (7 x 7,
+  // 13..14 x 13..14 at K = 5) always take it: 128x64x10x10 19 against 24 us.
+  const bool cl_tensor = ly.xs[1] == 1 && ly.ys[1] == 1 && ly.C > 1;
+  if (tune.cl >= 0 && cl_tensor && ly.stride == 1 && ly.L >= 1 && ly.L <= kPlanarMaxLev && (ly.K == 3 || ly.K == 5) &&
+      ly.H <= 64 && ly.W <= 64 && !regplane_supported(ly.K, ly.H, ly.W, ly.L)) {
+    const long long elements = (long long)ly.B * ly.C * ly.H * ly.W;
+    const bool narrow = ly.H <= 32 && ly.W <= 32;
+    const bool small_plane = ly.H <= 16 && ly.W <= 16 && !quad_supported(ly.K, ly.H, ly.W);
+    if (small_plane || elements <= (narrow ? 2000000 : 600000)) {
+      Stage2d st;
+      if (plan_planar(st.planar, ly, Hl.data(), Wl.data(), 0, ly.L, true, false, true, true) && st.planar.smem_bytes <= kSmemTwoPerSm) {
+        st.kind = 7;
+        st.xin_off = st.rin_off = st.rout_off = -1;
+        st.smem_bytes = st.planar.smem_bytes;
+        ch.stages.push_back(st);
+        return ch;
+      }
+    }
+  }
+
   // Bottom of the pyramid: when the plane of some level q is small enough for the
   // register-resident kernel (channels-last tensors, every remaining level), that kernel
   // takes levels q+1..L; the CTA-tile stages above it cover levels 1..q only.
@@ -696,7 +720,6 @@ inline Chain2d plan_layer(const Layer2d& ly, const Tuning2d& tune = Tuning2d()) 
   }
   // Kernel sizes 3, 5, 7 on every other tensor: the planar kernels.  (Channels-last tensors with K = 5 and
   // stride 1 that the kernels above do not take keep the register-level chain below.)
-  const bool cl_tensor = ly.xs[1] == 1 && ly.ys[1] == 1 && ly.C > 1;
   // A 7 x 7 plane fits a thread's registers whatever the layout (its loads then take a lane per plane, which
   // the caches absorb): in shared memory its frames and tap sets leave a quarter of the warps resident.
   const bool reg_whole = tune.cl >= 0 && !cl_tensor && ly.stride == 1 && ly.L >= 1 && regplane_supported(ly.K, ly.H, ly.W, ly.L);
