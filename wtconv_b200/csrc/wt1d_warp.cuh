@@ -21,9 +21,10 @@
 //
 // Samples enter and leave through a per-warp staging buffer, because a thread's run is SPT samples
 // apart from its neighbour's: 128-bit accesses straight to global memory at that distance took one
-// cycle of the load/store pipe per sector (the pipe was 75 % busy, DRAM 55 %).  Rows that start on a
-// 16-byte boundary are copied in with 16-byte cp.async, other fp32 rows with 4-byte ones.  The buffer is
-// swizzled (warp1d_slot) so that both sides of the exchange are free of bank conflicts.
+// cycle of the load/store pipe per sector (the pipe was 75 % busy, DRAM 55 %).  All copies are 16-byte
+// cp.async and 16-byte stores on aligned addresses, whatever element a row starts on: the buffer of such a
+// row is staged some elements late and shifted back in registers (an odd number of 16-bit rows word by word: 45 us
+// for 16 M samples).  The buffer is swizzled so that both sides of the exchange are free of bank conflicts.
 //
 // wt1d_wgrad_kernel (parameter gradients) runs the same cascade on the input and on the output
 // gradient at once and keeps every correlation sum of a channel in registers.
@@ -109,21 +110,26 @@ __device__ __forceinline__ void warp1d_copy16(void* dst, const void* src, int by
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
 }
 
-// Rows that do not start on a 16-byte boundary: a stream of aligned words of WB bytes from `base`, `late` elements
-// before the row; bytes past the row arrive as zeros.  (Not unrolled whole: the copy appears twice in a kernel
-// and the code must fit the instruction cache.)
-template <typename T, int SPT, int WB>
-__device__ __forceinline__ void warp1d_stream(const T* __restrict__ base, int late, int tw, int lane, int N, unsigned char* st) {
-  constexpr int CPT = SPT * (int)sizeof(T) / 16;
-  constexpr int EPW = WB / (int)sizeof(T), WPC = 16 / WB;           // elements per word, words per chunk
-#pragma unroll 8
-  for (int k = 0; k < SPT / EPW; ++k) {
-    const int word = lane + 32 * k, t = tw + word * EPW;            // element of `base`
-    const int left = (N + late - t) * (int)sizeof(T);               // bytes up to the end of the row
-    const int n = (t >= 0 && left > 0) ? imin(left, WB) : 0;
-    unsigned char* d = st + warp1d_own<T, SPT>(word / (WPC * CPT), (word / WPC) & (CPT - 1)) + (word & (WPC - 1)) * WB;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"((unsigned)__cvta_generic_to_shared(d)),
-                 "l"(n ? base + t : base), "n"(WB), "r"(n) : "memory");
+// Elements between the 16-byte boundary below an address and the address
+template <typename T>
+__device__ __forceinline__ int warp1d_late(const T* p) { return (int)((reinterpret_cast<uintptr_t>(p) & 15) / sizeof(T)); }
+
+// w[i] = the words of the stream that starts `sh` elements (less than a chunk, the same for the whole warp) into w
+template <typename T, int NW>
+__device__ __forceinline__ void warp1d_shift(unsigned (&w)[NW + 4], int sh) {
+  constexpr int EPW = 4 / (int)sizeof(T);
+  const int ws = sh / EPW;
+  if (ws & 2) {
+#pragma unroll
+    for (int i = 0; i < NW + 2; ++i) w[i] = w[i + 2];
+  }
+  if (ws & 1) {
+#pragma unroll
+    for (int i = 0; i < NW + 1; ++i) w[i] = w[i + 1];
+  }
+  if (EPW == 2 && (sh & 1)) {
+#pragma unroll
+    for (int i = 0; i < NW; ++i) w[i] = __funnelshift_r(w[i], w[i + 1], 16);
   }
 }
 
@@ -133,30 +139,23 @@ __device__ __forceinline__ void warp1d_stream(const T* __restrict__ base, int la
 template <typename T, int SPT>
 __device__ __forceinline__ void warp1d_fetch(const T* __restrict__ xr, int tw, int lane, int N, int up, unsigned char* st) {
   constexpr int VEC = 16 / (int)sizeof(T), CPT = SPT / VEC;
-  if (up == 1 && (reinterpret_cast<uintptr_t>(xr) & 15) == 0) {   // warp-uniform
-    const T* p = xr + tw + lane * VEC;
-    if (tw >= 0 && tw + 32 * SPT <= N) {                          // the whole span is inside the signal
+  if (up == 1) {
+    // chunks of the aligned stream that starts `late` elements before the row
+    const int late = warp1d_late(xr);
+    const T* base = xr - late;
+    const T* p = base + tw + lane * VEC;
+    if (tw >= 0 && tw + 32 * SPT + VEC <= N + late) {             // the whole span is inside the row
 #pragma unroll
       for (int k = 0; k < CPT; ++k) async_copy16(st + warp1d_line<T, SPT>(lane, k), p + 32 * VEC * k);
+      if (lane == 0) async_copy16(st + 32 * SPT * sizeof(T), p + 32 * SPT);      // the chunk behind the last run
     } else {
 #pragma unroll
-      for (int k = 0; k < CPT; ++k) {
+      for (int k = 0; k <= CPT; ++k) {
         const int t = tw + (lane + 32 * k) * VEC;
-        const int n = (t >= 0 && t < N) ? imin(N - t, VEC) * (int)sizeof(T) : 0;      // bytes inside the signal
-        warp1d_copy16(st + warp1d_line<T, SPT>(lane, k), n ? p + 32 * VEC * k : xr, n);
+        const int n = (t >= 0 && t < N + late) ? imin(N + late - t, VEC) * (int)sizeof(T) : 0;      // bytes up to the end of the row
+        if (k < CPT) warp1d_copy16(st + warp1d_line<T, SPT>(lane, k), n ? p + 32 * VEC * k : base, n);
+        else if (lane == 0) warp1d_copy16(st + 32 * SPT * sizeof(T), n ? p + 32 * SPT : base, n);
       }
-    }
-  } else if (up == 1 && (reinterpret_cast<uintptr_t>(xr) & 7) == 0) {
-    warp1d_stream<T, SPT, 8>(xr, 0, tw, lane, N, st);
-  } else if (up == 1) {
-    // A 16-bit row that starts in the middle of a word is staged one element late (warp1d_read shifts it back)
-    const int late = (int)((reinterpret_cast<uintptr_t>(xr) & 3) / sizeof(T));
-    warp1d_stream<T, SPT, 4>(xr - late, late, tw, lane, N, st);
-    if (sizeof(T) == 2 && lane == 0) {                              // the word behind the last run
-      const int t = tw + 32 * SPT, left = (N + late - t) * (int)sizeof(T);
-      const int n = (late && t >= 0 && left > 0) ? imin(left, 4) : 0;
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(st + 32 * SPT * sizeof(T))),
-                   "l"(n ? xr - late + t : xr - late), "r"(n) : "memory");
     }
   } else {
     const unsigned limit = (unsigned)(N / up * up);
@@ -171,31 +170,29 @@ __device__ __forceinline__ void warp1d_fetch(const T* __restrict__ xr, int tw, i
   }
 }
 
-// This thread's run, which starts at sample tw + lane * SPT; late: in the middle of its first word (16-bit types)
+// This thread's run, which starts at sample tw + lane * SPT and `late` elements into its place in the buffer
 template <typename T, int SPT>
-__device__ __forceinline__ void warp1d_read(const unsigned char* st, int lane, int tw, bool late, float (&v)[SPT]) {
+__device__ __forceinline__ void warp1d_read(const unsigned char* st, int lane, int tw, int late, float (&v)[SPT]) {
   constexpr int VEC = 16 / (int)sizeof(T), CPT = SPT / VEC;
-  if (sizeof(T) == 2 && late) {
-    unsigned w[4 * CPT + 1];
+  unsigned w[4 * CPT + 4];
 #pragma unroll
-    for (int k = 0; k < CPT; ++k) {
-      const uint4 q = *reinterpret_cast<const uint4*>(st + warp1d_own<T, SPT>(lane, k));
-      w[4 * k] = q.x; w[4 * k + 1] = q.y; w[4 * k + 2] = q.z; w[4 * k + 3] = q.w;
-    }
-    w[4 * CPT] = *reinterpret_cast<const unsigned*>(lane == 31 ? st + 32 * SPT * sizeof(T) : st + warp1d_own<T, SPT>(lane + 1, 0));
+  for (int k = 0; k < CPT; ++k) {
+    const uint4 q = *reinterpret_cast<const uint4*>(st + warp1d_own<T, SPT>(lane, k));
+    w[4 * k] = q.x; w[4 * k + 1] = q.y; w[4 * k + 2] = q.z; w[4 * k + 3] = q.w;
+  }
+  if (late) {                                                      // warp-uniform
+    const uint4 q = *reinterpret_cast<const uint4*>(lane == 31 ? st + 32 * SPT * sizeof(T) : st + warp1d_own<T, SPT>(lane + 1, 0));
+    w[4 * CPT] = q.x; w[4 * CPT + 1] = q.y; w[4 * CPT + 2] = q.z; w[4 * CPT + 3] = q.w;
+    warp1d_shift<T, 4 * CPT>(w, late);
+    if (tw + lane * SPT < 0) {                                     // the first chunk of a row also holds elements before it
 #pragma unroll
-    for (int k = 0; k < 4 * CPT; ++k) {
-      Chunk<T, 4> ch;
-      ch.raw = __funnelshift_r(w[k], w[k + 1], 16);
-      v[(2 * k) % SPT] = Elem<T>::to_f(ch.get(0)); v[(2 * k + 1) % SPT] = Elem<T>::to_f(ch.get(1 % ch.VEC));
+      for (int i = 0; i < 4 * CPT; ++i) w[i] = 0u;
     }
-    if (tw + (lane + 1) * SPT == 0) v[SPT - 1] = 0.f;              // the row's first word also holds the element before it
-    return;
   }
 #pragma unroll
   for (int k = 0; k < CPT; ++k) {
     Chunk<T, 16> ch;
-    ch.raw = *reinterpret_cast<const uint4*>(st + warp1d_own<T, SPT>(lane, k));
+    ch.raw = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
 #pragma unroll
     for (int i = 0; i < VEC; ++i) v[k * VEC + i] = Elem<T>::to_f(ch.get(i));
   }
@@ -286,7 +283,7 @@ wt1d_warp_kernel(const __grid_constant__ Warp1dArgs a) {
     __syncwarp();
     float xv[SPT];
     const T* xrow = static_cast<const T*>(a.x) + cur.n * a.xs0 + cur.c * a.xs1;
-    warp1d_read<T, SPT>(st, lane, cur.tw, a.up == 1 && (reinterpret_cast<uintptr_t>(xrow) & 3), xv);
+    warp1d_read<T, SPT>(st, lane, cur.tw, a.up == 1 ? warp1d_late(xrow) : 0, xv);
     const float* wch = reinterpret_cast<const float*>(st + BUF);
 
     // ---- levels, deepest first (recursion), then the base convolution and the bias
@@ -354,28 +351,30 @@ wt1d_warp_kernel(const __grid_constant__ Warp1dArgs a) {
               if (t + i < a.N) yr[t + i] = ch.get(i);
           }
         }
-      } else if (sizeof(T) == 2) {
-        // word by word: elements (2i - late, 2i - late + 1) of the segment
-        const int late = (int)((reinterpret_cast<uintptr_t>(yr) & 3) / 2);
-        auto at = [&](int idx) { return *(reinterpret_cast<const T*>(st + warp1d_own<T, SPT>(idx / SPT, (idx / VEC) & (CPT - 1))) + (idx & (VEC - 1))); };
-#pragma unroll 8
-        for (int k = 0; k <= SPT / 2; ++k) {
-          const int idx = 2 * (lane + 32 * k) - late + HL * SPT, t = cur.tw + idx;
-          const bool in0 = idx >= HL * SPT && idx < (32 - HL) * SPT && t < a.N;
-          const bool in1 = idx + 1 < (32 - HL) * SPT && t + 1 < a.N;
-          if (in0 && in1) {
-            Chunk<T, 4> ch;
-            ch.set(0, at(idx)); ch.set(1 % ch.VEC, at(idx + 1));
-            *reinterpret_cast<unsigned*>(yr + t) = ch.raw;
-          } else if (in0) yr[t] = at(idx);
-          else if (in1 && idx + 1 >= HL * SPT) yr[t + 1] = at(idx + 1);
-        }
       } else {
-#pragma unroll 8
-        for (int k = 0; k < SPT; ++k) {
-          const int idx = lane + 32 * k, t = cur.tw + idx;
-          if (idx >= HL * SPT && idx < (32 - HL) * SPT && t < a.N)
-            yr[t] = *(reinterpret_cast<const T*>(st + warp1d_own<T, SPT>(idx / SPT, (idx / VEC) & (CPT - 1))) + (idx & (VEC - 1)));
+        // aligned chunks of the row: each takes the end of one staged chunk and the start of the next
+        const int late = warp1d_late(yr);
+#pragma unroll 2
+        for (int k = 0; k <= CPT; ++k) {
+          const int q = HL * CPT - 1 + lane + 32 * k;              // staged chunk the aligned one starts in
+          if (q >= (32 - HL) * CPT) continue;
+          const int idx = q * VEC + VEC - late, t = cur.tw + idx;  // its first staged element and sample
+          unsigned w[8];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int c = imin(imax(q + h, 0), 32 * CPT - 1);
+            const uint4 v = *reinterpret_cast<const uint4*>(st + warp1d_own<T, SPT>(c / CPT, c & (CPT - 1)));
+            w[4 * h] = v.x; w[4 * h + 1] = v.y; w[4 * h + 2] = v.z; w[4 * h + 3] = v.w;
+          }
+          warp1d_shift<T, 4>(w, VEC - late);
+          Chunk<T, 16> ch;
+          ch.raw = make_uint4(w[0], w[1], w[2], w[3]);
+          if (idx >= HL * SPT && idx + VEC <= (32 - HL) * SPT && t + VEC <= a.N) *reinterpret_cast<uint4*>(yr + t) = ch.raw;
+          else {
+#pragma unroll
+            for (int i = 0; i < VEC; ++i)
+              if (idx + i >= HL * SPT && idx + i < (32 - HL) * SPT && t + i < a.N) yr[t + i] = ch.get(i);
+          }
         }
       }
     }
@@ -474,8 +473,8 @@ wt1d_wgrad_kernel(const __grid_constant__ Wgrad1dArgs a) {
     const int n = (int)(it / a.nseg), tw = (int)(it - (long long)n * a.nseg) * SEG - HL * SPT;
     const T* xr = static_cast<const T*>(a.x) + n * a.xs0 + c * a.xs1;
     const T* gr = static_cast<const T*>(a.g) + n * a.gs0 + c * a.gs1;
-    warp1d_read<T, SPT>(st + cur * 2 * BUF, lane, tw, reinterpret_cast<uintptr_t>(xr) & 3, xv);
-    warp1d_read<T, SPT>(st + cur * 2 * BUF + BUF, lane, tw, a.up == 1 && (reinterpret_cast<uintptr_t>(gr) & 3), gv);
+    warp1d_read<T, SPT>(st + cur * 2 * BUF, lane, tw, warp1d_late(xr), xv);
+    warp1d_read<T, SPT>(st + cur * 2 * BUF + BUF, lane, tw, a.up == 1 ? warp1d_late(gr) : 0, gv);
 #pragma unroll
     for (int o = 0; o < SPT; ++o) {                    // the outer lanes' positions belong to the neighbouring segments
       gv[o] = owner ? gv[o] : 0.f;
