@@ -201,10 +201,10 @@ inline long long plan_quad(QuadPlane& a, int B, int C, int K, int L, int q, int 
   a.wlen = ts * (a.has_base + 4);
   a.wpad = a.wlen + (((a.wlen / 4) % 2 == 0) ? 4 : 0);
   a.ngroups = cdiv(C, 32);
-  // about one wave of CTAs (three per SM): the tap sets are staged once per CTA
-  const long long tasks = (long long)B * a.ngroups;
-  a.samples_per_cta = (int)imax(1, (int)((tasks + 443) / 444));
-  a.nbatch = cdiv(B, a.samples_per_cta);
+  // one wave of CTAs (three per SM), each with every nbatch-th sample: the tap sets are staged once per CTA and
+  // the SMs end up with equal shares
+  a.nbatch = imin(B, imax(1, 444 / a.ngroups));
+  a.samples_per_cta = cdiv(B, a.nbatch);
   const long long chlast[4] = {(long long)C * Hp * Wp, 1, (long long)Wp * C, C};
   const long long rcl[4] = {(long long)C * kQuadP * kQuadP, 1, (long long)kQuadP * C, C};
   for (int i = 0; i < 4; ++i) {

@@ -80,7 +80,7 @@ WT_HD void quad_cta(const QuadPlane& a, const T* __restrict__ x, T* __restrict__
   }
 
   for (int it = 0; it < a.samples_per_cta; ++it) {
-    const int n = nb * a.samples_per_cta + it;
+    const int n = nb + it * a.nbatch;               // strided: the CTAs of a group differ by one sample at most
     if (n >= a.B) break;                            // uniform over the CTA
 
     // ---- phase 1: polyphase component of the plane -> XS
