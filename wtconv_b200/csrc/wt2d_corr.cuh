@@ -47,6 +47,49 @@ __device__ __forceinline__ void planar_corr(const float* __restrict__ p, int pit
   }
 }
 
+// 4 x 4 pixels in their own type, 16-bit ones two to a register; rows at and beyond `nrow` and columns outside
+// [0, W) are zero
+template <typename T>
+struct GradQuad {
+  static constexpr int EPW = 4 / (int)sizeof(T);
+  unsigned w[16 / EPW];
+  __device__ __forceinline__ void load(const T* __restrict__ p, int x, int W, int s2, int s3, bool wide, int nrow) {
+#pragma unroll
+    for (int i = 0; i < 16 / EPW; ++i) w[i] = 0u;
+    if (wide) {
+      typedef typename RawChunk<4 * (int)sizeof(T)>::type raw_t;
+      union { raw_t raw[4]; unsigned u[16 / EPW]; } v;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        v.raw[i] = raw_t();
+        if (i < nrow && x < W) v.raw[i] = __ldg(reinterpret_cast<const raw_t*>(p + i * s2 + x));
+      }
+#pragma unroll
+      for (int i = 0; i < 16 / EPW; ++i) w[i] = v.u[i];
+      return;
+    }
+    const T* q = p + x * s3;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (!(i < nrow && x + k < W)) continue;
+        Chunk<T, 4> c;
+        c.raw = w[(4 * i + k) / EPW];
+        c.set(k % EPW, q[i * s2 + k * s3]);
+        w[(4 * i + k) / EPW] = c.raw;
+      }
+  }
+  __device__ __forceinline__ void widen(float (&v)[4][4]) const {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      Chunk<T, 4> c;
+      c.raw = w[i / EPW];
+      v[i / 4][i % 4] = Elem<T>::to_f(c.get(i % EPW));
+    }
+  }
+};
+
 // Transpose of planar_synthesis: lane t = 2 ty + tx of a tile holds its 4 x 4 pixel quadrant; afterwards lane s
 // holds the un-normalised sub-band s at the tile's 4 x 4 positions.
 __device__ __forceinline__ void planar_split(const float (&o)[4][4], float (&v)[4][4], int lane) {
@@ -96,10 +139,28 @@ wt2d_corr_kernel(const __grid_constant__ PlanarStage p, const __grid_constant__ 
 #pragma unroll
   for (int k = 0; k < KK; ++k) { accs[k] = 0.f; if (BASE) accb[BASE ? k : 0] = 0.f; }
   const int per = p.nty * p.ntx, items = p.B * per;
+  const bool wide = a.gvec >= 4 && p.w[0] % 4 == 0;
   for (int item = split; item < items; item += a.nsplit) {
     const int n = item / per, t2 = item - n * per;
     const int tile_y = t2 / p.ntx, tile_x = t2 - tile_y * p.ntx;
     const int Y0 = tile_y * p.TH, X0 = tile_x * p.TW;
+    // tiles of the item that lie on the plane
+    const int tyn = imin(p.tyn[1], (p.h[1] - Y0 + 3) >> 2), txn = imin(p.txn[1], (p.w[1] - X0 + 3) >> 2);
+    const int ntile = tyn * txn, slots = (ntile + tpw - 1) >> (3 - gpl);
+    const float inv = 1.f / (float)txn;
+    // K = 7 (one CTA per SM, registers to spare): the gradient pixels of a slot are requested one slot ahead, those
+    // of the first before the frames are filled.  (32x96x40x40 step 312 -> 287 us; with two CTAs per SM
+    // at K = 5 the registers cost more than the wait, 477 -> 488 us.)
+    constexpr bool AHEAD = K == 7;
+    GradQuad<T> gq;
+    auto request = [&](int slot) {
+      const int tq = (slot << (3 - gpl)) + (u >> gpl), t = imin(tq, ntile - 1);
+      const int ty = planar_div(t, inv), tx = t - ty * txn;
+      const int yy = 2 * Y0 + 8 * ty + 4 * (s >> 1), xx = 2 * X0 + 8 * tx + 4 * (s & 1);
+      const T* gp = gy + (long long)n * a.gs[0] + (long long)(c0 + g) * a.gs[1] + (long long)yy * a.gs[2];
+      gq.load(gp, xx, p.w[0], (int)a.gs[2], (int)a.gs[3], wide, slot < slots && tq < ntile && g < gc ? p.h[0] - yy : 0);
+    };
+    if (AHEAD) request(warp);
     {
       PlanarFill<T, K, BASE, 0> f{p, sm, x + (long long)n * p.xs[0] + (long long)c0 * p.xs[1], gc, Y0 - HS, X0 - HS, 0, 0, 0, 0, 0.f};
       if (p.tiled) { f.rb = 4 * p.tyn[1] + 2 * HS; f.cb = 4 * p.txn[1] + 2 * HS; }
@@ -108,10 +169,6 @@ wt2d_corr_kernel(const __grid_constant__ PlanarStage p, const __grid_constant__ 
       f.run(tid, nthr);
     }
     __syncthreads();
-    // tiles of the item that lie on the plane
-    const int tyn = imin(p.tyn[1], (p.h[1] - Y0 + 3) >> 2), txn = imin(p.txn[1], (p.w[1] - X0 + 3) >> 2);
-    const int ntile = tyn * txn, slots = (ntile + tpw - 1) >> (3 - gpl);
-    const float inv = 1.f / (float)txn;
 #pragma unroll 1
     for (int slot = warp; slot < slots; slot += nwarp) {
       const int tq = (slot << (3 - gpl)) + (u >> gpl), t = imin(tq, ntile - 1);
@@ -119,28 +176,9 @@ wt2d_corr_kernel(const __grid_constant__ PlanarStage p, const __grid_constant__ 
       const int ty = planar_div(t, inv), tx = t - ty * txn;
       const int qy = 8 * ty + 4 * (s >> 1), qx = 8 * tx + 4 * (s & 1);      // this lane's pixel quadrant in the frame
       float q4[4][4];
-      {
-        const int yy = 2 * Y0 + qy, xx = 2 * X0 + qx;
-        const T* gp = gy + (long long)n * a.gs[0] + (long long)(c0 + g) * a.gs[1] + (long long)yy * a.gs[2];
-        const int W = p.w[0];
-        if (a.gvec >= 4 && W % 4 == 0) {
-          PlanarQuad<T, 4> r[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) r[i].load(gp + i * (int)a.gs[2], xx, W, 1, live && yy + i < p.h[0]);
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) q4[i][q] = r[i].get(q);
-        } else {
-          PlanarQuad<T, 1> r[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) r[i].load(gp + i * (int)a.gs[2], xx, W, (int)a.gs[3], live && yy + i < p.h[0]);
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) q4[i][q] = r[i].get(q);
-        }
-      }
+      if (!AHEAD) request(slot);
+      gq.widen(q4);
+      if (AHEAD) request(slot + nwarp);
       if constexpr (BASE) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) sum += (q4[i][0] + q4[i][1]) + (q4[i][2] + q4[i][3]);

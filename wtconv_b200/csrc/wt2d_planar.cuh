@@ -276,24 +276,33 @@ struct PlanarFill {
     const PlanarWalk wk(ncols, tid, nthr);
     const int nr = rb - ra, nrows = nch * nr;
     const int s2 = (int)p.xs[2], s3 = (int)p.xs[3], splane = p.splane[1];
-    for (int row = wk.row; row < nrows; row += wk.step) {
+    // With four chunks per position the next one's are on their way while a position is worked on (a thread then
+    // waits for memory once per column, not once per position); the sixteen of SHIFT = 1 fill the registers.
+    Chunk<T, CB> ahead[SHIFT ? 1 : NP][SHIFT ? 1 : NP];
+    auto fetch = [&](auto& q, int row, int c) {
       const int ch = planar_div(row, inv_nr), r = ra + row - ch * nr;          // chunk slowest: a warp covers neighbouring pixels
-      const int y = NP * (py0 + r);
-      for (int c = ca + wk.col; c < cb; c += 32) {
-        const int x = NP * (px0 + c);
-        Chunk<T, CB> q[NP][NP];
-        {
-          const T* q0 = src + (y * s2 + x * s3 + ch * V);
-          const bool inside = y >= 0 && x >= 0 && y + NP <= H && x + NP <= W;
+      const int y = NP * (py0 + r), x = NP * (px0 + c);
+      const T* q0 = src + (y * s2 + x * s3 + ch * V);
+      const bool inside = y >= 0 && x >= 0 && y + NP <= H && x + NP <= W;
 #pragma unroll
-          for (int dy = 0; dy < NP; ++dy)
+      for (int dy = 0; dy < NP; ++dy)
 #pragma unroll
-            for (int dx = 0; dx < NP; ++dx) {
-              q[dy][dx].raw = raw_t();                          // zero bits are 0.0 in every type
-              if (inside || (y + dy >= 0 && y + dy < H && x + dx >= 0 && x + dx < W))
-                q[dy][dx].raw = __ldg(reinterpret_cast<const raw_t*>(q0 + dy * s2 + dx * s3));
-            }
+        for (int dx = 0; dx < NP; ++dx) {
+          q[dy][dx].raw = raw_t();                              // zero bits are 0.0 in every type
+          if (row < nrows && (inside || (y + dy >= 0 && y + dy < H && x + dx >= 0 && x + dx < W)))
+            q[dy][dx].raw = __ldg(reinterpret_cast<const raw_t*>(q0 + dy * s2 + dx * s3));
         }
+    };
+    for (int c = ca + wk.col; c < cb; c += 32) {
+      if constexpr (SHIFT == 0) fetch(ahead, wk.row, c);
+      for (int row = wk.row; row < nrows; row += wk.step) {
+        const int ch = planar_div(row, inv_nr), r = ra + row - ch * nr;
+        Chunk<T, CB> q[NP][NP];
+        if constexpr (SHIFT == 0) {
+#pragma unroll
+          for (int k = 0; k < NP * NP; ++k) q[k / NP][k % NP].raw = ahead[k / NP][k % NP].raw;
+          fetch(ahead, row + wk.step, c);
+        } else fetch(q, row, c);
         const int fr = 2 * r - HS, fc = 2 * c - HS;             // first pixel in the pixel frame
         const bool c0 = FINAL && fc >= 0 && fc < p.xcols, c1 = FINAL && fc + 1 >= 0 && fc + 1 < p.xcols;
         const bool r0 = fr >= 0 && fr < p.xrows, r1 = fr + 1 >= 0 && fr + 1 < p.xrows;
