@@ -149,6 +149,28 @@ struct PlanarWalk {
   }
 };
 
+// The same with as many rows per pass as fit the threads, for the fill: frames with their halo are just wider than a
+// power of two (20 positions of a 16-wide tile), which left a third of the lanes idle.  Set up once per fill.
+struct PlanarPack {
+  int col, row, step, cstep;
+  __device__ __forceinline__ PlanarPack(int ncols, int nrows, int tid, int nthr) {
+    if (ncols >= nthr) { col = tid; row = 0; step = 1; cstep = nthr; return; }
+    cstep = ncols;
+    const int sh = 32 - __clz(ncols - 1 > 0 ? ncols - 1 : 0);
+    if (8 * ncols >= (7 << sh)) {                      // close to a power of two: no division
+      col = tid & ((1 << sh) - 1);
+      row = col < ncols ? tid >> sh : nrows;
+      step = nthr >> sh;
+      return;
+    }
+    const float inv = 1.f / (float)ncols;
+    step = planar_div(nthr, inv);
+    row = planar_div(tid, inv);
+    col = tid - row * ncols;
+    if (row >= step) row = nrows;                      // left over
+  }
+};
+
 // Fill of a CTA's planes: pixels -> pixel frame (with the base path) and sub-bands of the first level.
 // (ra, rb) x (ca, cb): rows and columns of the sub-band frame to write; frame cell (r, c) is position
 // (py0 + r, px0 + c) of level 1, its pixels rows 2r - HS, 2r - HS + 1 of the pixel frame.
@@ -178,13 +200,13 @@ struct PlanarFill {
   __device__ __forceinline__ void rows(int tid, int nthr) const {
     const int H = p.Hsrc, W = p.Wsrc;
     const int ncols = (cb - ca + 1) / 2, nr = rb - ra;
-    const PlanarWalk wk(ncols, tid, nthr);
     const int nrows = gc * nr;
+    const PlanarPack wk(ncols, nrows, tid, nthr);
     const int g0 = planar_div(wk.row, inv_nr), r0 = wk.row - g0 * nr;
     const int dg = planar_div(wk.step, inv_nr), dr = wk.step - dg * nr;
     const int s1 = (int)p.xs[1], s2 = (2 << SHIFT) * (int)p.xs[2];              // source steps of a channel and of a position row
     const int splane = p.splane[1], spitch = p.spitch[1];
-    for (int ci = wk.col; ci < ncols; ci += 32) {
+    for (int ci = wk.col; ci < ncols; ci += wk.cstep) {
       const int c = ca + 2 * ci, x = (2 << SHIFT) * (px0 + c);
       const bool two = c + 1 < cb;
       int r = r0, y = (2 << SHIFT) * (py0 + ra + r0);
@@ -273,8 +295,8 @@ struct PlanarFill {
     typedef typename RawChunk<CB>::type raw_t;
     const int H = p.Hsrc, W = p.Wsrc;
     const int nch = p.G / V, ncols = cb - ca;
-    const PlanarWalk wk(ncols, tid, nthr);
     const int nr = rb - ra, nrows = nch * nr;
+    const PlanarPack wk(ncols, nrows, tid, nthr);
     const int s2 = (int)p.xs[2], s3 = (int)p.xs[3], splane = p.splane[1];
     // With four chunks per position the next one's are on their way while a position is worked on (a thread then
     // waits for memory once per column, not once per position); the sixteen of SHIFT = 1 fill the registers.
@@ -293,7 +315,7 @@ struct PlanarFill {
             q[dy][dx].raw = __ldg(reinterpret_cast<const raw_t*>(q0 + dy * s2 + dx * s3));
         }
     };
-    for (int c = ca + wk.col; c < cb; c += 32) {
+    for (int c = ca + wk.col; c < cb; c += wk.cstep) {
       if constexpr (SHIFT == 0) fetch(ahead, wk.row, c);
       for (int row = wk.row; row < nrows; row += wk.step) {
         const int ch = planar_div(row, inv_nr), r = ra + row - ch * nr;
