@@ -26,6 +26,9 @@
 // row is staged some elements late and shifted back in registers (an odd number of 16-bit rows word by word: 45 us
 // for 16 M samples).  The buffer is swizzled so that both sides of the exchange are free of bank conflicts.
 //
+// (512,64,4096) fp32, four levels: 281 us before the staging and the copy one item ahead, 225 us with them, 4.8 TB/s; bound
+// by DRAM (73 % of the copy rate) with the issue slots 69 % busy.
+//
 // wt1d_wgrad_kernel (parameter gradients) runs the same cascade on the input and on the output
 // gradient at once and keeps every correlation sum of a channel in registers.
 #pragma once

@@ -11,24 +11,6 @@ namespace wt {
 
 namespace {
 
-// Launch with or without the programmatic-dependent-launch attribute (the kernel then calls
-// griddepcontrol.wait before it reads what the preceding kernel of the stream wrote)
-template <typename Kern, typename... Args>
-cudaError_t launch_maybe_dependent(Kern kern, dim3 grid, int threads, size_t smem, cudaStream_t stream, bool dependent,
-                                   const Args&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = dependent ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

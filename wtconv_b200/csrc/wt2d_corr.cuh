@@ -3,7 +3,8 @@
 //
 // The kernels of wt2d_wgrad.cuh wrote both pyramids to memory in fp32 (one launch per level and tensor) and
 // read every window from there, lanes over channels (stage-1 layer at batch 64: 130 us of pyramids and 187 us of
-// sums for 1.1 G multiply-adds, 32 us at the FP32 rate).  Here
+// sums for 1.1 G multiply-adds, 32 us at the FP32 rate; now 160 + 38 + 30 us, bound by the latency of the fill and by the
+// issue slots, half busy).  Here
 //
 //   * wt2d_corr_kernel takes one level (and the base path with the first): the input's frames are filled as
 //     in wt2d_planar.cuh, and a lane again owns one sub-band of a 4 x 4 tile.  The gradient never enters

@@ -22,8 +22,10 @@ cudaError_t launch_inst(const QuadPlane& a, const void* x, void* y, const float*
   cudaError_t e = allow_full_smem(kern, done);
   if (e != cudaSuccess) return e;
   const dim3 blocks((unsigned)a.ngroups, (unsigned)a.nbatch);
-  kern<<<blocks, kQuadThreads, smem_bytes, stream>>>(a, static_cast<const T*>(x), static_cast<T*>(y), rin, rout, packed);
-  return cudaGetLastError();
+  // a programmatic dependent of the kernel that writes `rin`; it reads x directly only in two-kernel-deep chains whose first
+  // launch is an ordinary one
+  return launch_maybe_dependent(kern, blocks, kQuadThreads, smem_bytes, stream, a.has_base != 0, a, static_cast<const T*>(x),
+                                static_cast<T*>(y), rin, rout, packed);
 }
 
 }  // namespace

@@ -119,6 +119,9 @@ WT_HD void quad_cta(const QuadPlane& a, const T* __restrict__ x, T* __restrict__
           }
       }
       if (a.has_rin) {
+        // from the launch before this one, which may still be running: by now the tap sets and the first
+        // sample's pixels are on chip (128x384x14x14: 67.9 -> 65.6 us a call)
+        wait_for_producer();
         const float* rp = rin + (long long)n * a.rs[0] + (long long)c * a.rs[1];
         const int rs2 = (int)a.rs[2], rs3 = (int)a.rs[3];
         for (int e = q; e < P * P; e += 4) RS[e * 32 + lane] = rp[(e / P) * rs2 + (e % P) * rs3];

@@ -22,8 +22,8 @@ cudaError_t launch_inst(const RegPlane& a, const void* x, void* y, float* rout, 
   cudaError_t e = allow_full_smem(kern, done);
   if (e != cudaSuccess) return e;
   const dim3 blocks((unsigned)a.ngroups, (unsigned)a.nbatch);
-  kern<<<blocks, kRegPlaneThreads, smem_bytes, stream>>>(a, static_cast<const T*>(x), static_cast<T*>(y), rout, packed);
-  return cudaGetLastError();
+  return launch_maybe_dependent(kern, blocks, kRegPlaneThreads, smem_bytes, stream, !BASE, a, static_cast<const T*>(x),
+                                static_cast<T*>(y), rout, packed);
 }
 
 template <typename T, bool BASE>

@@ -145,6 +145,7 @@ WT_HD void regplane_cta(const RegPlane& a, const T* __restrict__ x, T* __restric
   constexpr int TS = TapSet2d<K>::value;
   const int nthr = kRegPlaneThreads;
   const int c0 = cg * 32;
+  launch_dependents();
 
   // ---- tap sets of the 32 channels -> shared memory (pitch wpad: odd multiple of 16 bytes,
   //      so the 128-bit reads of a quarter warp fall into eight different bank groups)
@@ -158,6 +159,7 @@ WT_HD void regplane_cta(const RegPlane& a, const T* __restrict__ x, T* __restric
     async_wait_all();
   }
 
+  if (!BASE) wait_for_producer();                   // the low-pass planes come from the launch before this one
   WT_PHASE(nthr) {
     const int lane = tid & 31, warp = tid >> 5;
     const int c = c0 + lane;

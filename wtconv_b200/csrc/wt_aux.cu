@@ -57,6 +57,7 @@ template <typename T>
 __global__ void reduce_planes_kernel(const T* __restrict__ in, float* __restrict__ out, int B, int C, int Hin,
                                      int Win, int Hout, int Wout, int shift, long long s0, long long s1,
                                      long long s2, long long s3, int out_cl) {
+  launch_dependents();
   const long long total = (long long)B * C * Hout * Wout;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x)
@@ -70,6 +71,7 @@ template <typename T>
 __global__ void reduce_planes_cl_kernel(const T* __restrict__ in, float* __restrict__ out, int B, int C, int Hin,
                                         int Win, int Hout, int Wout, int shift, long long s0, long long s2,
                                         long long s3, int out_cl) {
+  launch_dependents();
   constexpr int V = 16 / (int)sizeof(T);
   const int chunks = C / V;
   const int edge = 1 << shift;

@@ -91,6 +91,18 @@ WT_HD void async_copy4_zfill(void* smem_dst, const void* gmem_src, bool valid) {
   *static_cast<unsigned int*>(smem_dst) = valid ? *static_cast<const unsigned int*>(gmem_src) : 0u;
 #endif
 }
+// Programmatic dependent launch: lets the next kernel of the stream start / waits until the preceding one has
+// completed and its writes are visible (nothing for kernels launched without the attribute)
+WT_HD void launch_dependents() {
+#ifdef __CUDA_ARCH__
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
+WT_HD void wait_for_producer() {
+#ifdef __CUDA_ARCH__
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
+}
 WT_HD void async_wait_all() {
 #ifdef __CUDA_ARCH__
   asm volatile("cp.async.wait_all;" ::: "memory");
@@ -114,6 +126,24 @@ inline cudaError_t allow_full_smem(Kern kern, bool (&done)[kMaxDevices]) {
   e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynamicSmem);
   if (e == cudaSuccess) __atomic_store_n(&done[dev], true, __ATOMIC_RELEASE);
   return e;
+}
+
+// Launch with or without the programmatic-dependent-launch attribute (the kernel then calls
+// griddepcontrol.wait before it reads what the preceding kernel of the stream wrote)
+template <typename Kern, typename... Args>
+inline cudaError_t launch_maybe_dependent(Kern kern, dim3 grid, int threads, size_t smem, cudaStream_t stream, bool dependent,
+                                   const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = dependent ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 #endif
 
