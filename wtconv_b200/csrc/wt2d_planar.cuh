@@ -3,7 +3,7 @@
 //
 // Replaces, for the planes of a CTA, wtconv/wtconv2d.py:46-85.  The tile kernels of wt2d_fused.cuh that did
 // this before spent 290 thread instructions per element on a path of 58 multiply-adds (28 x 28 planes, K = 5:
-// 125 us for 6.4 M elements, FMA pipe 21 % busy; now 53 us, 170 instructions, 39 %); what was changed and why:
+// 125 us for 6.4 M elements, FMA pipe 21 % busy; now 53 us, 180 instructions, 38 %); what was changed and why:
 //
 //   * everything is planar fp32 in shared memory with zero borders that are cleared once: CTAs are
 //     persistent and later planes rewrite the interior only;
