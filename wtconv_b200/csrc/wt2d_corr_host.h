@@ -97,6 +97,9 @@ inline CorrChain plan_corr(const Layer2d& ly) {          // ly.ys / y_align: the
     in = st.out_off;
     const long long items = (long long)st.p.B * st.p.nty * st.p.ntx;
     long long split = 148LL * resident(st.p) / st.p.ngroups;
+    // one-warp CTAs (planes of one tile: nothing waits at a barrier; 256x768x7x7 step 304 -> 248 us): at least four items
+    // each, because 5 (K*K + 1) sums per channel end as atomics
+    if (split > (items + 3) / 4 && st.p.nthreads == 32) split = (items + 3) / 4;
     if (split > items) split = items;
     st.nsplit = (int)(split < 1 ? 1 : split);
     if ((long long)st.nsplit * st.p.ngroups >= (1LL << 31) || items >= (1LL << 31)) { ch.status = -6; return ch; }

@@ -43,7 +43,7 @@ struct PlanarStage {
 
 inline int planar_resident(const PlanarStage& p) {          // CTAs per SM
   const int by_smem = (228 * 1024) / (p.smem_bytes + 1024), by_regs = p.ctas * kPlanarMaxThreads / p.nthreads;
-  return imax(1, imin(by_smem, by_regs));
+  return imax(1, imin(imin(by_smem, by_regs), 32));
 }
 
 // Fills the geometry of a stage; returns its dynamic shared memory in bytes.
@@ -114,7 +114,7 @@ inline long long planar_layout(PlanarStage& p) {
   const int slots = (p.G / gp) * cdiv(p.tyn[1] * p.txn[1], tpw);
   int best = 2, warps = 0;
   p.score = 0.0;
-  for (int nw = kPlanarMaxThreads / 32; nw >= 2; --nw) {
+  for (int nw = kPlanarMaxThreads / 32; nw >= (p.frames_only ? 1 : 2); --nw) {   // gradients of one-tile planes: a warp alone, no barrier to wait at
     p.nthreads = 32 * nw;
     const int resident = planar_resident(p);
     const double per_sm = (double)p.total / 148.0;
